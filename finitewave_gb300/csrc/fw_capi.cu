@@ -105,6 +105,12 @@ int check_step_args(const fw_step_args *a, int64_t n_steps)
             set_error("fw_step: state variable %d is NULL", i);
             return FW_ERR_ARG;
         }
+    if (a->node_list && (a->n_list_myo < 0 ||
+                         a->n_list_myo > a->ni * a->nj * a->nk ||
+                         a->ni * a->nj * a->nk > INT32_MAX)) {
+        set_error("fw_step: node_list needs 0 <= n_list_myo <= N < 2^31");
+        return FW_ERR_ARG;
+    }
     if (a->n_stims < 0 || a->n_stims > FW_MAX_STIMS || a->n_at < 0 ||
         a->n_at > FW_MAX_AT || a->n_lat < 0 || a->n_lat > FW_MAX_LAT ||
         a->n_probe < 0 || a->n_probe > FW_MAX_PROBE) {
@@ -278,6 +284,12 @@ int fw_ionic(int32_t model, int32_t precision, void *u_new, const void *u,
         }
     return fw::ionic(model, precision, u_new, u, state, idx, n_idx, dt, params,
                      (cudaStream_t)stream);
+}
+
+int fw_node_list(const int8_t *myo, int64_t n, int32_t *list, int32_t *scratch,
+                 void *stream)
+{
+    return fw::node_list(myo, n, list, scratch, (cudaStream_t)stream);
 }
 
 int fw_pack_weights(int32_t stencil, const float *w, int64_t n, float *out,

@@ -184,6 +184,8 @@ int ecg(int32_t stencil, int32_t precision, const void *u, const void *w,
         cudaStream_t stream);
 int step_fused(const fw_step_args *a, int64_t n_begin, int64_t n_steps,
                cudaStream_t stream);
+int node_list(const int8_t *myo, int64_t n, int32_t *list, int32_t *scratch,
+              cudaStream_t stream);
 int pack_weights(int32_t stencil, const float *w, int64_t n, float *out,
                  cudaStream_t stream);
 int step_fused_ap(const fw_step_args *a, int64_t n_begin, int64_t n_steps,

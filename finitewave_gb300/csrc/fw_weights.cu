@@ -458,4 +458,105 @@ int build_weights(int32_t stencil, int32_t precision, const int8_t *mesh,
     return FW_OK;
 }
 
+// ---- node list ---------------------------------------------------------------
+// Stable partition of the nodes by the myocyte flag, once per tissue: per-CTA
+// counts, one CTA's scan of them, and the placement.
+namespace {
+
+constexpr int kListThreads = 256, kListChunk = 4096;
+
+__global__ void __launch_bounds__(kListThreads)
+    k_list_count(const int8_t *__restrict__ myo, int64_t n, int32_t *count)
+{
+    const int64_t p0 = blockIdx.x * (int64_t)kListChunk;
+    int c = 0;
+    for (int q = threadIdx.x; q < kListChunk; q += kListThreads)
+        c += p0 + q < n && myo[p0 + q];
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
+    __shared__ int s[kListThreads / 32];
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int t = 0;
+        for (int w = 0; w < kListThreads / 32; ++w) t += s[w];
+        count[blockIdx.x] = t;
+    }
+}
+
+// Inclusive scan over the CTA's kListThreads values.
+__device__ __forceinline__ int block_scan(int v, int *s)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += t;
+    }
+    if (lane == 31) s[warp] = v;
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) v += s[w];
+    __syncthreads();
+    return v;
+}
+
+// count[0 .. nb) -> exclusive sums, count[nb] = the total
+__global__ void __launch_bounds__(kListThreads) k_list_scan(int32_t *count, int nb)
+{
+    __shared__ int s[kListThreads / 32];
+    __shared__ int last;
+    int base = 0;
+    for (int b0 = 0; b0 < nb; b0 += kListThreads) {
+        const int b = b0 + threadIdx.x;
+        const int v = b < nb ? count[b] : 0;
+        const int incl = block_scan(v, s);
+        if (b < nb) count[b] = base + incl - v;
+        if (threadIdx.x == kListThreads - 1) last = incl;
+        __syncthreads();
+        base += last;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) count[nb] = base;
+}
+
+__global__ void __launch_bounds__(kListThreads)
+    k_list_write(const int8_t *__restrict__ myo, int64_t n,
+                 const int32_t *__restrict__ count, int32_t *__restrict__ list)
+{
+    __shared__ int s[kListThreads / 32];
+    __shared__ int last;
+    const int64_t p0 = blockIdx.x * (int64_t)kListChunk;
+    const int64_t n_myo = count[gridDim.x];
+    int64_t before = count[blockIdx.x];   // myocytes before this round's nodes
+    for (int q0 = 0; q0 < kListChunk; q0 += kListThreads) {
+        const int64_t p = p0 + q0 + threadIdx.x;
+        const int m = p < n && myo[p] ? 1 : 0;
+        const int incl = block_scan(m, s);
+        const int64_t mb = before + incl - m;   // myocytes before p
+        if (p < n) list[m ? mb : n_myo + (p - mb)] = (int32_t)p;
+        if (threadIdx.x == kListThreads - 1) last = incl;
+        __syncthreads();
+        before += last;
+        __syncthreads();
+    }
+}
+
+}  // namespace
+
+int node_list(const int8_t *myo, int64_t n, int32_t *list, int32_t *scratch,
+              cudaStream_t stream)
+{
+    if (!myo || !list || !scratch || n < 1 || n > INT32_MAX) {
+        set_error("fw_node_list: null pointer, or a grid of %lld nodes",
+                  (long long)n);
+        return FW_ERR_ARG;
+    }
+    const int nb = (int)((n + kListChunk - 1) / kListChunk);
+    k_list_count<<<nb, kListThreads, 0, stream>>>(myo, n, scratch);
+    FW_CHECK_LAUNCH("k_list_count");
+    k_list_scan<<<1, kListThreads, 0, stream>>>(scratch, nb);
+    FW_CHECK_LAUNCH("k_list_scan");
+    k_list_write<<<nb, kListThreads, 0, stream>>>(myo, n, scratch, list);
+    FW_CHECK_LAUNCH("k_list_write");
+    return FW_OK;
+}
+
 }  // namespace fw

@@ -316,6 +316,24 @@ class CardiacModel:
             self._step_stencil = _ffi.ANISO19_XY
         self._pack_weights()
         self._weight_rows()
+        self._node_order()
+
+    def _node_order(self):
+        """The nodes with the myocytes first (fw_step_args.node_list), for
+        the plain steps that run one thread per myocyte: float64 and the
+        detailed models."""
+        self._nodes = None
+        if (self._precision() == _ffi.F32 and
+                self._model_id not in self._DETAILED_MODELS):
+            return
+        n = self._myo_d.numel()
+        if n < 1 << 31:
+            dev = self._myo_d.device
+            self._nodes = torch.empty(n, dtype=torch.int32, device=dev)
+            scratch = torch.empty(n // 4096 + 2, dtype=torch.int32, device=dev)
+            _ffi.call("fw_node_list", self._myo_d.data_ptr(), n,
+                      self._nodes.data_ptr(), scratch.data_ptr(),
+                      torch.cuda.current_stream().cuda_stream)
 
     def _weight_rows(self, force=False):
         """FW_STENCIL_ANISO19_XY steps read the eleven weight planes 0-8,
@@ -531,6 +549,7 @@ class CardiacModel:
         n_seg = int(np.argmax(stop)) + 1 if stop.any() else limit
         return ts_all[:n_seg], float(ts_all[n_seg]), n_seg
 
+    _DETAILED_MODELS = (_ffi.MODEL_TP06, _ffi.MODEL_CRN, _ffi.MODEL_LR91)
     _FUSED_MODELS = (_ffi.MODEL_AP, _ffi.MODEL_MS, _ffi.MODEL_FK,
                      _ffi.MODEL_BK)
 
@@ -627,6 +646,10 @@ class CardiacModel:
             if self._wrows is not None and a.stencil == _ffi.ANISO19_XY:
                 a.weight_rows = self._wrows.data_ptr()
                 a.weight_row_index = self._widx.data_ptr()
+        nodes = getattr(self, "_nodes", None)
+        if nodes is not None:
+            a.node_list = nodes.data_ptr()
+            a.n_list_myo = self._n_myo
         wpack = getattr(self, "_wpack", None)
         a.weights_packed = wpack.data_ptr() if wpack is not None else None
         a.u[0] = self._dev["u"].data_ptr()

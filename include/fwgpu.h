@@ -325,6 +325,14 @@ typedef struct fw_step_args {
                             the step reads these instead of `weights`
                             (same values, same sums).  NULL otherwise      */
     const int32_t *weight_row_index; /* (N) row of each node, or NULL    */
+    const int32_t *node_list; /* plain form, optional (NULL: none): a
+                            permutation of the N < 2^31 nodes with the
+                            n_list_myo nodes of myo == 1 first, each part
+                            in ascending order.  The steps whose cost is
+                            arithmetic (float64, the detailed models) then
+                            run one thread per myocyte, so no lane of a
+                            warp idles on a non-myocyte; same results       */
+    int64_t n_list_myo;
 } fw_step_args;
 
 /* A planned batch of tissues (fw_batch_plan).  Host-side handle; the
@@ -411,6 +419,12 @@ FW_API int fw_diffuse(int32_t stencil, int32_t precision, void *u_new, const voi
 FW_API int fw_ionic(int32_t model, int32_t precision, void *u_new, const void *u,
              void *const *state, const int64_t *idx, int64_t n_idx,
              double dt, const double *params, void *stream);
+
+/* fw_step_args.node_list of a grid: the n < 2^31 nodes with those of
+ * myo != 0 first, each part in ascending order, written to list (n).
+ * scratch: device int32, n / 4096 + 2 values. */
+FW_API int fw_node_list(const int8_t *myo, int64_t n, int32_t *list,
+             int32_t *scratch, void *stream);
 
 /* Repack float32 weight-major weights (nw, N) into the node-major layout of
  * the fused TMA kernel: out[p * nwo + q] = w[plane_q * N + p] over the

@@ -1,0 +1,78 @@
+"""GPU: the myocytes-first node list of the plain form (fw_node_list) and
+the listed steps against the grid-order steps, bit for bit."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def fg():
+    if not torch.cuda.is_available():
+        pytest.fail("CUDA device required for -m gpu tests")
+    import finitewave_gb300 as fg
+    return fg
+
+
+# sizes around the warp, the scan's CTA and its 4096-node chunk
+@pytest.mark.parametrize("n", [1, 31, 33, 256, 4095, 4096, 4097, 12289, 2500000])
+@pytest.mark.parametrize("p", [0.0, 0.3, 1.0])
+def test_node_list(fg, n, p):
+    gen = np.random.default_rng(n)
+    myo = (gen.random(n) < p).astype(np.int8)
+    d = torch.as_tensor(myo, device="cuda")
+    out = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    scratch = torch.empty(n // 4096 + 2, dtype=torch.int32, device="cuda")
+    fg._ffi.call("fw_node_list", d.data_ptr(), n, out.data_ptr(),
+                 scratch.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    want = np.concatenate([np.flatnonzero(myo), np.flatnonzero(myo == 0)])
+    assert np.array_equal(out.cpu().numpy(), want)
+
+
+def _model(fg, cls, npfloat, shape, special):
+    gen = np.random.default_rng(3)
+    tissue = (fg.CardiacTissue2D if len(shape) == 2
+              else fg.CardiacTissue3D)(shape)
+    tissue.mesh = np.where(gen.random(shape) < 0.25, 2, 1).astype(np.int8)
+    if special:
+        tissue.special_boundaries = (gen.random(shape) < 0.1).astype(np.int8)
+    m = cls()
+    m.dt, m.dr, m.t_max, m.npfloat = 0.01, 0.25, 0.2, npfloat
+    m.form = "plain"
+    m.cardiac_tissue = tissue
+    seq = fg.StimSequence()
+    box = [b for n in shape for b in (0, n // 2)]
+    stim = fg.StimVoltageCoord2D if len(shape) == 2 else fg.StimVoltageCoord3D
+    seq.add_stim(stim(0.03, 20.0 if m._model_id in m._DETAILED_MODELS else 1.0,
+                      *box))
+    m.stim_sequence = seq
+    trs = fg.TrackerSequence()
+    for t in (fg.ActivationTime2DTracker(), fg.LocalActivationTime2DTracker()):
+        # the init potential is above one threshold and below the other, and
+        # one tracker starts late, so non-myocytes are tracked as well
+        t.threshold = -90.0 if m._model_id in m._DETAILED_MODELS else 0.5
+        trs.add_tracker(t)
+    trs.sequence[0].start_time = 0.05
+    m.tracker_sequence = trs
+    return m, trs.sequence
+
+
+@pytest.mark.parametrize("special", [False, True])
+@pytest.mark.parametrize("cls,npfloat,shape", [
+    ("AlievPanfilov2D", "float64", (137, 145)), ("FentonKarma3D", "float64", (29, 34, 21)),
+    ("TP062D", "float32", (133, 154)), ("Courtemanche3D", "float32", (27, 29, 33)),
+    ("LuoRudy912D", "float64", (120, 175))])
+def test_listed_steps_equal_grid_order(fg, cls, npfloat, shape, special):
+    out = []
+    for listed in (True, False):
+        m, trs = _model(fg, getattr(fg, cls), npfloat, shape, special)
+        m.initialize()
+        assert m._nodes is not None
+        if not listed:
+            m._nodes = None
+        m.run(initialize=False)
+        out.append([getattr(m, n) for n in ["u", "u_new"] + list(m._state_names)] +
+                   [t.output for t in trs])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
