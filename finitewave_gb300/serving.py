@@ -60,8 +60,6 @@ def device_footprint(model):
     per_node += nw * b
     if prec == _ffi.F32 and len(shape) == 2:
         per_node += (nw - 1) * 4                           # packed weights
-    if prec == _ffi.F64 or model._model_id in model._DETAILED_MODELS:
-        per_node += 4                                      # node order
     trs = model.tracker_sequence.sequence if model.tracker_sequence else []
     for tr in trs:
         name = type(tr).__name__
