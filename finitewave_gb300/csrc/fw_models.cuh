@@ -8,6 +8,8 @@
 //
 // Interface of a model M:
 //   M::NS, M::NP            number of state variables after u / parameters
+//   M::ND, M::derive(p, dt, q)  number of values derived from the parameters on
+//                           the host (q[NP .. NP + ND - 1]; ND = 0: none)
 //   M::St<T>                the node's state variables in registers
 //   M::load<T>(s, p)        read state of node p from the arrays s[0..NS-1]
 //   M::store<T>(s, p, x)    write it back
@@ -100,11 +102,21 @@ __device__ __forceinline__ Params<T, N> load_params(const S *p)
     return r;
 }
 
+// The parameters and what is derived from them, rounded to T (host).
+template <class M, class T>
+inline void fill_params(T *out, const double *params, double dt)
+{
+    double q[M::NP + M::ND];
+    for (int i = 0; i < M::NP; ++i) q[i] = params[i];
+    if constexpr (M::ND > 0) M::derive(params, dt, q);
+    for (int i = 0; i < M::NP + M::ND; ++i) out[i] = (T)q[i];
+}
+
 // Aliev-Panfilov.  params: a, k, eap, mu_1, mu_2 (aliev_panfilov_2d.py:
 // 290-295).  calc_v (:337-374), then the voltage update with the new v
 // (ionic_kernel_2d :376-406).
 struct ModelAP {
-    static constexpr int NS = 1, NP = 5;
+    static constexpr int NS = 1, NP = 5, ND = 0;
     template <class T>
     struct St {
         T v;
@@ -200,7 +212,7 @@ struct ModelAP {
 // (mitchell_schaeffer_2d.py:57-61).  calc_h, calc_J_in, calc_J_out,
 // ionic_kernel_2d (:102-217).  u**2 is u*u as numba compiles it.
 struct ModelMS {
-    static constexpr int NS = 1, NP = 5;
+    static constexpr int NS = 1, NP = 5, ND = 0;
     template <class T>
     struct St {
         T h;
@@ -248,7 +260,7 @@ struct ModelMS {
 // calc_v, calc_w, calc_Jfi, calc_Jso, calc_Jsi, ionic_kernel_2d (:143-328);
 // J_si takes the fast gate v, as the reference passes it (:326).
 struct ModelFK {
-    static constexpr int NS = 2, NP = 11;
+    static constexpr int NS = 2, NP = 11, ND = 0;
     template <class T>
     struct St {
         T v, w;
@@ -301,7 +313,7 @@ struct ModelFK {
 // signature :141); calc_v (:114-138) then the voltage update with the new v
 // (:141-170).
 struct ModelBK {
-    static constexpr int NS = 1, NP = 3;
+    static constexpr int NS = 1, NP = 3, ND = 0;
     template <class T>
     struct St {
         T v;
@@ -347,7 +359,7 @@ struct ModelBK {
 // w_inf_.  calc_v, calc_w, calc_s, J_fi, J_so, J_si with the updated gates
 // (ionic_kernel_2d, bueno_orovio_2d.py).
 struct ModelBO {
-    static constexpr int NS = 3, NP = 28;
+    static constexpr int NS = 3, NP = 28, ND = 0;
     enum {
         u_o, u_u, theta_v, theta_w, theta_v_m, theta_o, tau_v1_m, tau_v2_m,
         tau_v_p, tau_w1_m, tau_w2_m, k_w_m, u_w_m, tau_w_p, tau_fi, tau_o1,

@@ -80,7 +80,7 @@ struct LatK {
     int32_t cap;
 };
 
-template <class T>
+template <class M, class T>
 struct StepK {
     const int8_t *myo;
     const T *w;
@@ -90,8 +90,8 @@ struct StepK {
     const int32_t *widx;
     const T *u;
     T *un;
-    void *state[FW_MAX_STATE];
-    T params[FW_MAX_PARAMS];
+    void *state[M::NS];
+    T params[M::NP + M::ND];
     T dt;
     int64_t n, si, sj;
     // nodes in list order, myocytes first (NULL: every node in grid order);
@@ -112,8 +112,8 @@ __device__ __forceinline__ bool finite_bits(double x)
 }
 __device__ __forceinline__ bool finite_bits(float x) { return isfinite(x); }
 
-template <class T>
-__device__ __forceinline__ void track(const StepK<T> &k, int64_t p, T uc)
+template <class M, class T>
+__device__ __forceinline__ void track(const StepK<M, T> &k, int64_t p, T uc)
 {
     for (int a = 0; a < k.n_at; ++a) {
         // (act_t < 0) & (u > threshold)  (activation_time_2d_tracker.py:61-63)
@@ -190,9 +190,9 @@ constexpr int step_blocks()
 
 template <class M, int ST, class T, bool LIST>
 __global__ void __launch_bounds__(step_threads<T>(), (MinBlocks<M, T>::value))
-    k_step(StepK<T> k)
+    k_step(StepK<M, T> k)
 {
-    const Params<T, M::NP> P = load_params<T, M::NP>(k.params);
+    const Params<T, M::NP + M::ND> P = load_params<T, M::NP + M::ND>(k.params);
     const T dt = k.dt;
     const int64_t n = LIST ? (int64_t)k.n_run : k.n;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
@@ -475,8 +475,8 @@ template <class M, class T>
 struct IonicK {
     T *un;
     const T *u;
-    void *state[FW_MAX_STATE];
-    T params[FW_MAX_PARAMS];
+    void *state[M::NS];
+    T params[M::NP + M::ND];
     T dt;
     const int64_t *idx;
     int64_t n_idx;
@@ -485,7 +485,7 @@ struct IonicK {
 template <class M, class T>
 __global__ void k_ionic(IonicK<M, T> k)
 {
-    const Params<T, M::NP> P = load_params<T, M::NP>(k.params);
+    const Params<T, M::NP + M::ND> P = load_params<T, M::NP + M::ND>(k.params);
     const T dt = k.dt;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
          t < k.n_idx; t += (int64_t)gridDim.x * blockDim.x) {
@@ -540,7 +540,7 @@ int run_plain(const fw_step_args *a, int64_t n_begin, int64_t n_steps,
 {
     int dim = stencil_dim(ST);
     Grid g = make_grid(a->ni, a->nj, a->nk, dim);
-    StepK<T> k;
+    StepK<M, T> k;
     k.myo = a->myo;
     k.w = (const T *)a->weights;
     k.wrow = (const T *)a->weight_rows;
@@ -551,8 +551,8 @@ int run_plain(const fw_step_args *a, int64_t n_begin, int64_t n_steps,
                   "index and 16-byte aligned rows");
         return FW_ERR_ARG;
     }
-    for (int i = 0; i < FW_MAX_STATE; ++i) k.state[i] = a->state[i];
-    for (int i = 0; i < FW_MAX_PARAMS; ++i) k.params[i] = (T)a->params[i];
+    for (int i = 0; i < M::NS; ++i) k.state[i] = a->state[i];
+    fill_params<M, T>(k.params, a->params, a->dt);
     k.dt = (T)a->dt;
     k.n = g.n;
     k.si = g.si;
@@ -684,9 +684,8 @@ int run_ionic(void *u_new, const void *u, void *const *state,
     IonicK<M, T> k;
     k.un = (T *)u_new;
     k.u = (const T *)u;
-    for (int i = 0; i < FW_MAX_STATE; ++i) k.state[i] = i < M::NS ? state[i] : nullptr;
-    for (int i = 0; i < FW_MAX_PARAMS; ++i)
-        k.params[i] = i < M::NP ? (T)params[i] : (T)0;
+    for (int i = 0; i < M::NS; ++i) k.state[i] = state[i];
+    fill_params<M, T>(k.params, params, dt);
     k.dt = (T)dt;
     k.idx = idx;
     k.n_idx = n_idx;

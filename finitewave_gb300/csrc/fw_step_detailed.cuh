@@ -1,9 +1,9 @@
 // fw_step_detailed.cuh -- the plain form and the ionic pass of the detailed
 // models (TP06, Courtemanche) at one fixed precision.  Each model x precision
 // pair is its own translation unit (fw_step_detailed_*.cu): the expression
-// trees are large, so splitting keeps the build parallel, and the float64
-// units are compiled without FMA contraction (closest to the reference's
-// evaluation order) while the float32 units use FMA and fast division.
+// trees are large, so splitting keeps the build parallel.  The float64 units
+// are compiled with FMA contraction (a float64 step lasts as long as the
+// float64 instructions it issues), the float32 units with fast division too.
 #pragma once
 
 #include "fw_models_big.cuh"
