@@ -300,8 +300,8 @@ def run_batched(args, fg, torch, reps):
             "myocytes": sum(myo), "time_steps_per_bench_step": chunk,
             "bench_steps": k_b, "launches": int(launches),
             "ms_per_step": 1e3 * el / k_b,
-            "kernel": {"name": {1: "k_batch", 2: "k_batch_tma",
-                                3: "k_batch_tma (column pairs, f32x2)"}
+            "kernel": {"name": {1: "k_batch", 2: "k_batch_group / k_batch_all",
+                                3: "k_batch_group / k_batch_all (column pairs, f32x2)"}
                                [batch_kernel],
                        "value": kernel_value,
                        "ms_per_time_step": kms / chunk,

@@ -510,7 +510,7 @@ int64_t tissue_tiles(const fw_step_args *a)
 // TMA-read arrays.
 
 constexpr int kTmaR = 4;                           // rows per thread
-constexpr int kRun = 4;                            // tiles per counter claim
+constexpr int kRun = 4;                            // most tiles per counter claim
 constexpr int kTmaNT = fused::kTW * (LH / kTmaR);  // 512 threads
 
 struct alignas(128) BTissueT {
@@ -557,24 +557,24 @@ struct BatchTmaSmem {
 };
 
 // The batch's (model, stencil) groups, in the order the plan sorts tiles;
-// each group is advanced by its own instantiation of k_batch_tma.
+// each group is advanced by its own instantiation of batch_group.
 constexpr int kGroups = 6;
 constexpr int kGroupKey[kGroups] = {
     FW_MODEL_AP * 8 + FW_STENCIL_ISO5, FW_MODEL_AP * 8 + FW_STENCIL_ANISO9,
     FW_MODEL_MS * 8 + FW_STENCIL_ISO5, FW_MODEL_MS * 8 + FW_STENCIL_ANISO9,
     FW_MODEL_FK * 8 + FW_STENCIL_ISO5, FW_MODEL_FK * 8 + FW_STENCIL_ANISO9};
 
-// The per-launch fields of every tissue's launch description: step window
-// masks of the stimuli and trackers, first step, step count and the
-// potential buffers.  One warp per tissue.
-__global__ void k_batch_events(BTissueT *__restrict__ tissues, int32_t n,
-                               int64_t koff, int32_t ks, int32_t in_buf)
+// Time of a group's tile, in any unit (us measured with one group alone):
+// the groups' parts of the SMs follow it.
+constexpr double kGroupCost[kGroups] = {4.8, 5.0, 5.8, 6.3, 6.8, 7.1};
+
+// The per-launch fields of tissue T's launch description: step window masks
+// of the stimuli and trackers, first step, step count and the potential
+// buffers.  One warp.
+__device__ __forceinline__ void tissue_events(BTissueT &T, int lane, int64_t koff,
+                                              int32_t ks, int32_t in_buf)
 {
-    const int i = blockIdx.x * blockDim.y + threadIdx.y;
-    if (i >= n) return;
-    BTissueT &T = tissues[i];
     fused::FusedK &F = T.f;
-    const int lane = threadIdx.x;
     const int64_t n0 = T.step_base + koff;
     if (lane < F.n_stims)
         F.stims[lane].on =
@@ -601,6 +601,15 @@ __global__ void k_batch_events(BTissueT *__restrict__ tissues, int32_t n,
             F.state_out[q] = T.state[in_buf ^ 1][q];
         }
     }
+}
+
+// Before the first launch of a run; each launch's last CTA does it for the
+// next one.
+__global__ void k_batch_events(BTissueT *__restrict__ tissues, int32_t n,
+                               int64_t koff, int32_t ks, int32_t in_buf)
+{
+    const int i = blockIdx.x * blockDim.y + threadIdx.y;
+    if (i < n) tissue_events(tissues[i], threadIdx.x, koff, ks, in_buf);
 }
 
 __device__ __forceinline__ void tensormap_acquire(const void *map)
@@ -761,26 +770,22 @@ __device__ __noinline__ void batch_issue_split(const BTissueT *__restrict__ tiss
     }
 }
 
-// One (model, stencil) group of the batch: tiles [t_begin, t_end) of the
-// list, claimed kRun at a time from counters[0] (counters[1] counts the
-// CTAs that are done; the last one zeroes both).  PAIR (kernel 3): the tile
-// code of the column-pair kernels in two-wide float32 instructions
-// (tma_tile2), 2 x 2 nodes per thread, the same bits as the strip tiles.
+// The CTA's part of one (model, stencil) group of the batch: tiles [t_begin,
+// t_end) of the list, claimed `run` at a time from *counter.  PAIR (kernel
+// 3): the tile code of the column-pair kernels in two-wide float32
+// instructions (tma_tile2), 2 x 2 nodes per thread, the same bits as the
+// strip tiles.
 template <class M, int ST, bool PAIR>
-__global__ void __launch_bounds__(kTmaNT, 1)
-    k_batch_tma(const BTissueT *__restrict__ tissues, const BTileT *__restrict__ tiles,
-                int32_t t_begin, int32_t t_end, int32_t n_tissues, int32_t in_buf,
-                uint32_t *counters)
+__device__ __forceinline__ void batch_group(const BTissueT *__restrict__ tissues,
+                                        const BTileT *__restrict__ tiles,
+                                        int32_t t_begin, int32_t t_end,
+                                        int32_t n_tissues, int32_t in_buf,
+                                        int32_t run, uint32_t *counter,
+                                        unsigned char *smem)
 {
     using Sm = BatchTmaSmem<M::NS, fused::Stencil2D<ST>::NWO>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const unsigned mis = fused::smem_u32(smem_raw) & 127u;
-    Sm &S = *reinterpret_cast<Sm *>(smem_raw + (mis ? 128u - mis : 0u));
+    Sm &S = *reinterpret_cast<Sm *>(smem);
     const int tid = threadIdx.x;
-    // the next group's kernel, launched with programmatic serialisation,
-    // may place its CTAs on the SMs this grid's CTAs leave (its tissues are
-    // not this group's, so nothing it reads is written here)
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     uint32_t own_c, ring_c;
     if constexpr (PAIR)
         fused::pair_masks<KMAX, LH>(2 * (tid % (fused::kTW / 2)),
@@ -789,34 +794,37 @@ __global__ void __launch_bounds__(kTmaNT, 1)
         fused::strip_masks<KMAX, LH, kTmaR>(tid % fused::kTW,
                                             (tid / fused::kTW) * kTmaR, own_c, ring_c);
     const BTileT none{-1, -1, 0, 0};
-    // thread 0's tiles: runs of kRun consecutive list entries (mostly of
+    // thread 0's tiles: runs of `run` consecutive list entries (mostly of
     // one tissue), each
-    // run's start taken from counters[0] one run ahead; the list entry of
+    // run's start taken from the counter one run ahead; the list entry of
     // tile i + 1 is read while tile i is computed
     int run_cur = t_end, run_end = t_end, run_next = t_end;
     auto take_run = [&]() -> int {
         const int64_t s =
-            (int64_t)t_begin + (int64_t)atomicAdd(&counters[0], 1u) * kRun;
+            (int64_t)t_begin + (int64_t)atomicAdd(counter, 1u) * run;
         return s < t_end ? (int)s : t_end;
     };
     auto next_tile = [&]() -> int {
         if (run_cur >= run_end) {
             if (run_next >= t_end) return t_end;
             run_cur = run_next;
-            run_end = run_next + kRun < t_end ? run_next + kRun : t_end;
+            run_end = run_next + run < t_end ? run_next + run : t_end;
             run_next = take_run();
         }
         return run_cur++;
     };
     int t_next = t_end;
     BTileT b_next = none;
+    for (int i = tid; i < 4 * kAcq; i += kTmaNT) {
+        if (i < kAcq) S.acq[i] = -1;
+        else S.acq3[i / kAcq - 1][i % kAcq] = -1;
+    }
+    __syncthreads();
     if (tid == 0) {
         fused::mbar_init(&S.t.bar[0], 1);
         fused::mbar_init(&S.t.bar[1], 1);
         fused::mbar_fence_init();
         S.ftissue[0] = S.ftissue[1] = -1;
-        for (int i = 0; i < kAcq; ++i) S.acq[i] = -1;
-        for (int i = 0; i < 3 * kAcq; ++i) S.acq3[i / kAcq][i % kAcq] = -1;
         run_next = take_run();
         const int t0 = next_tile();
         t_next = next_tile();
@@ -883,7 +891,25 @@ __global__ void __launch_bounds__(kTmaNT, 1)
         // that record, and the next iteration's wait ends in one before any
         // thread touches the ping-pong rows or this stage is refilled
     }
-    if (tid == 0) {
+}
+
+// Large batches (kGroupKernels): one kernel per group, launched one after
+// the other.
+template <class M, int ST, bool PAIR>
+__global__ void __launch_bounds__(kTmaNT, 1)
+    k_batch_group(const BTissueT *__restrict__ tissues, const BTileT *__restrict__ tiles,
+                  int32_t t_begin, int32_t t_end, int32_t n_tissues, int32_t in_buf,
+                  int32_t run, uint32_t *counters)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const unsigned mis = fused::smem_u32(smem_raw) & 127u;
+    // the next group's kernel, launched with programmatic serialisation,
+    // may place its CTAs on the SMs this grid's CTAs leave (its tissues are
+    // not this group's, so nothing it reads is written here)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    batch_group<M, ST, PAIR>(tissues, tiles, t_begin, t_end, n_tissues, in_buf, run,
+                             &counters[0], smem_raw + (mis ? 128u - mis : 0u));
+    if (threadIdx.x == 0) {
         // this grid completes only after the group's kernel launched before
         // it (a no-op without programmatic serialisation), so the stream's
         // next ordinary launch finds every group of the launch finished
@@ -896,6 +922,70 @@ __global__ void __launch_bounds__(kTmaNT, 1)
     }
 }
 
+// Other batches: one launch for all groups.  CTAs first[g] .. first[g + 1] -
+// 1 take group g's tiles, as many as the group's part of the work, and the
+// CTA that is done last fills the next launch's events.  With a kernel per
+// group, a small batch's time was the six kernels' start-up (each about 6 us
+// before its first tile) and their launches one behind the other; one
+// kernel holds six copies of the tile loop at 128 registers, of which the
+// Fenton-Karma ones spill a few (5 % slower a tile), hence the other form
+// for large batches.  One launch of four steps, measured (CUDA events):
+//   tiles        121   1016   1963   3436   28677
+//   per group   39.2   88.9  137.0  192.8   975.8 us
+//   one kernel  21.2   54.6   91.3  171.6  1035.0 us
+struct BatchK {
+    BTissueT *tissues;
+    const BTileT *tiles;
+    uint32_t *scratch;              // [1]: CTAs done; [2 + 2 g]: group g's tiles
+    int32_t n_tissues, in_buf;
+    int32_t first[kGroups + 1];     // CTAs
+    int32_t tile_end[kGroups];      // cumulative tiles
+    int32_t run[kGroups];           // tiles per counter claim
+    int64_t next_koff;              // the next launch's events (ks 0: none)
+    int32_t next_ks;
+};
+
+template <bool PAIR>
+__global__ void __launch_bounds__(kTmaNT, 1) k_batch_all(const __grid_constant__ BatchK k)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const unsigned mis = fused::smem_u32(smem_raw) & 127u;
+    unsigned char *smem = smem_raw + (mis ? 128u - mis : 0u);
+    int g = 0;
+    while (g < kGroups - 1 && (int)blockIdx.x >= k.first[g + 1]) ++g;
+#define FW_BATCH_GROUP(GI, M, ST)                                                 \
+    case GI:                                                                      \
+        batch_group<M, ST, PAIR>(k.tissues, k.tiles, GI ? k.tile_end[GI - 1] : 0, \
+                                 k.tile_end[GI], k.n_tissues, k.in_buf,           \
+                                 k.run[GI], k.scratch + 2 + 2 * GI, smem);        \
+        break;
+    switch (g) {
+        FW_BATCH_GROUP(0, ModelAP, FW_STENCIL_ISO5)
+        FW_BATCH_GROUP(1, ModelAP, FW_STENCIL_ANISO9)
+        FW_BATCH_GROUP(2, ModelMS, FW_STENCIL_ISO5)
+        FW_BATCH_GROUP(3, ModelMS, FW_STENCIL_ANISO9)
+        FW_BATCH_GROUP(4, ModelFK, FW_STENCIL_ISO5)
+        FW_BATCH_GROUP(5, ModelFK, FW_STENCIL_ANISO9)
+    }
+#undef FW_BATCH_GROUP
+    // the last CTA to finish zeroes the counters and fills the next
+    // launch's events (no CTA reads a description any more)
+    unsigned *done = reinterpret_cast<unsigned *>(smem);   // the stages are free
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        *done = atomicAdd(&k.scratch[1], 1u);
+    }
+    __syncthreads();
+    if (*done != gridDim.x - 1) return;
+    if (threadIdx.x < kGroups) atomicExch(&k.scratch[2 + 2 * threadIdx.x], 0u);
+    if (threadIdx.x == 0) atomicExch(&k.scratch[1], 0u);
+    if (k.next_ks)
+        for (int i = threadIdx.x / 32; i < k.n_tissues; i += kTmaNT / 32)
+            tissue_events(k.tissues[i], threadIdx.x % 32, k.next_koff, k.next_ks,
+                          k.in_buf ^ 1);
+}
+
 template <class M, int ST>
 constexpr size_t tma_smem()
 {
@@ -905,12 +995,13 @@ static_assert(tma_smem<ModelFK, FW_STENCIL_ANISO9>() <= 232448,
               "the batched TMA stages exceed 227 KB");
 
 using BatchTmaKernel = void (*)(const BTissueT *, const BTileT *, int32_t, int32_t,
-                                int32_t, int32_t, uint32_t *);
+                                int32_t, int32_t, int32_t, uint32_t *);
 
 inline int batch_group_launch_k(BatchTmaKernel kern, size_t smem, bool attr_only,
                                 cudaLaunchConfig_t &cfg, const BTissueT *desc,
                                 const BTileT *tl, int32_t t_begin, int32_t t_end,
-                                int32_t n_tissues, int32_t in_buf, uint32_t *counters)
+                                int32_t n_tissues, int32_t in_buf, int32_t run,
+                                uint32_t *counters)
 {
     if (attr_only) {
         FW_CUDA_CHECK(cudaFuncSetAttribute(
@@ -919,8 +1010,8 @@ inline int batch_group_launch_k(BatchTmaKernel kern, size_t smem, bool attr_only
     }
     cfg.dynamicSmemBytes = smem;
     FW_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, desc, tl, t_begin, t_end, n_tissues,
-                                     in_buf, counters));
-    FW_CHECK_LAUNCH("k_batch_tma");
+                                     in_buf, run, counters));
+    FW_CHECK_LAUNCH("k_batch_group");
     return FW_OK;
 }
 
@@ -932,7 +1023,7 @@ inline int batch_group_launch_k(BatchTmaKernel kern, size_t smem, bool attr_only
 inline int batch_group_launch(int g, bool pair, bool attr_only, bool overlap, int grid,
                               const BTissueT *desc, const BTileT *tl, int32_t t_begin,
                               int32_t t_end, int32_t n_tissues, int32_t in_buf,
-                              uint32_t *counters, cudaStream_t stream)
+                              int32_t run, uint32_t *counters, cudaStream_t stream)
 {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -946,13 +1037,13 @@ inline int batch_group_launch(int g, bool pair, bool attr_only, bool overlap, in
 #define FW_BATCH_GROUP(GI, M, ST)                                                 \
     case GI:                                                                      \
         if (pair)                                                                 \
-            return batch_group_launch_k(k_batch_tma<M, ST, true>,                 \
+            return batch_group_launch_k(k_batch_group<M, ST, true>,               \
                                         tma_smem<M, ST>(), attr_only, cfg, desc,  \
                                         tl, t_begin, t_end, n_tissues, in_buf,    \
-                                        counters);                                \
-        return batch_group_launch_k(k_batch_tma<M, ST, false>, tma_smem<M, ST>(), \
+                                        run, counters);                              \
+        return batch_group_launch_k(k_batch_group<M, ST, false>, tma_smem<M, ST>(), \
                                     attr_only, cfg, desc, tl, t_begin, t_end,     \
-                                    n_tissues, in_buf, counters);
+                                    n_tissues, in_buf, run, counters);
     switch (g) {
         FW_BATCH_GROUP(0, ModelAP, FW_STENCIL_ISO5)
         FW_BATCH_GROUP(1, ModelAP, FW_STENCIL_ANISO9)
@@ -965,6 +1056,25 @@ inline int batch_group_launch(int g, bool pair, bool attr_only, bool overlap, in
     set_error("fw_batch: no group %d", g);
     return FW_ERR_ARG;
 }
+
+constexpr size_t kTmaSmem = tma_smem<ModelFK, FW_STENCIL_ANISO9>();   // the largest
+
+// Shared-memory attributes of the kernels.
+inline int batch_tma_attr(bool pair, cudaStream_t stream)
+{
+    FW_CUDA_CHECK(cudaFuncSetAttribute(pair ? k_batch_all<true> : k_batch_all<false>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)kTmaSmem));
+    for (int g = 0; g < kGroups; ++g) {
+        int rc = batch_group_launch(g, pair, true, false, 0, nullptr, nullptr, 0, 0, 0, 0,
+                                    0, nullptr, stream);
+        if (rc) return rc;
+    }
+    return FW_OK;
+}
+
+// Tiles per CTA from which a batch runs one kernel per group.
+constexpr int kGroupKernels = 64;
 
 static_assert(sizeof(fused::FusedK) % 16 == 0 && offsetof(BTissueT, f) % 16 == 0,
               "the launch description moves as one bulk copy");
@@ -1267,11 +1377,8 @@ int batch_plan(const fw_step_args *const *tissues, int32_t n,
     FW_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     if (kernel >= 2) {
         // one persistent CTA per SM (the stages fill its shared memory)
-        for (int g = 0; g < kGroups; ++g) {
-            int rc2 = batch_group_launch(g, kernel == 3, true, false, 0, nullptr,
-                                         nullptr, 0, 0, 0, 0, nullptr, stream);
-            if (rc2) return rc2;
-        }
+        int rc2 = batch_tma_attr(kernel == 3, stream);
+        if (rc2) return rc2;
         per_sm = 1;
     } else {
         FW_CUDA_CHECK(cudaFuncSetAttribute(
@@ -1300,6 +1407,43 @@ int batch_plan(const fw_step_args *const *tissues, int32_t n,
     return FW_OK;
 }
 
+namespace batch {
+
+// CTAs of each group's kernel and tiles per counter claim.
+inline void group_shares(const fw_batch &b, int *grid, int *run)
+{
+    double total = 0.0, w[kGroups];
+    int32_t begin = 0, groups = 0;
+    for (int g = 0; g < kGroups; ++g) {
+        w[g] = kGroupCost[g] * (b.group_end[g] - begin);
+        groups += w[g] > 0;
+        total += w[g];
+        begin = b.group_end[g];
+    }
+    int left = b.grid;
+    begin = 0;
+    for (int g = 0; g < kGroups; ++g) {
+        const int n = b.group_end[g] - begin;
+        begin = b.group_end[g];
+        grid[g] = run[g] = 0;
+        if (n <= 0) continue;
+        // of the CTAs not given out yet, this group's part of the work not
+        // given out yet, at least one CTA for each group to come
+        --groups;
+        int k = (int)(left * (w[g] / total) + 0.5);
+        if (k > left - groups) k = left - groups;
+        if (k < 1) k = 1;
+        if (k > n) k = n;
+        left -= k;
+        total -= w[g];
+        grid[g] = k;
+        const int r = n / (4 * k);
+        run[g] = r < 1 ? 1 : r > kRun ? kRun : r;
+    }
+}
+
+}  // namespace batch
+
 int batch_run(const fw_batch *b, uint32_t *scratch, int64_t offset,
               int64_t n_steps, cudaStream_t stream)
 {
@@ -1322,11 +1466,8 @@ int batch_run(const fw_batch *b, uint32_t *scratch, int64_t offset,
     FW_CUDA_CHECK(cudaStreamIsCapturing(stream, &cap));
     if (cap == cudaStreamCaptureStatusNone) {
         if (tma) {
-            for (int g = 0; g < kGroups; ++g) {
-                int rc = batch_group_launch(g, pair, true, false, 0, nullptr, nullptr, 0,
-                                            0, 0, 0, nullptr, stream);
-                if (rc) return rc;
-            }
+            int rc = batch_tma_attr(pair, stream);
+            if (rc) return rc;
         } else {
             FW_CUDA_CHECK(cudaFuncSetAttribute(
                 k_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
@@ -1339,6 +1480,23 @@ int batch_run(const fw_batch *b, uint32_t *scratch, int64_t offset,
         (const unsigned char *)b->plan + align_up(desc_bytes * b->n_tissues, 256);
     const BTile *tl = reinterpret_cast<const BTile *>(tiles_dev);
     const BTileT *tl_t = reinterpret_cast<const BTileT *>(tiles_dev);
+    BatchK k;
+    int grid = 0;
+    const bool by_group = tma && b->n_tiles >= (int64_t)kGroupKernels * b->grid;
+    if (tma && !by_group) {
+        k.tissues = desc_t;
+        k.tiles = tl_t;
+        k.scratch = scratch;
+        k.n_tissues = b->n_tissues;
+        int grids[kGroups];
+        group_shares(*b, grids, k.run);
+        for (int g = 0; g < kGroups; ++g) {
+            k.first[g] = grid;
+            grid += grids[g];
+            k.tile_end[g] = b->group_end[g];
+        }
+        k.first[kGroups] = grid;
+    }
     // L launches of <= KMAX steps with L == n_steps (mod 2): the result ends
     // in u[(offset + n_steps) & 1], as after the same steps of the plain form
     int64_t L = (n_steps + KMAX - 1) / KMAX;
@@ -1350,27 +1508,39 @@ int batch_run(const fw_batch *b, uint32_t *scratch, int64_t offset,
         if (ks > KMAX) ks = KMAX;
         const int in_buf = (int)((offset + li) & 1);
         if (tma) {
-            const dim3 eb(32, 4);
-            k_batch_events<<<(unsigned)((b->n_tissues + 3) / 4), eb, 0, stream>>>(
-                desc_t, b->n_tissues, offset + done, (int32_t)ks, in_buf);
-            FW_CHECK_LAUNCH("k_batch_events");
-            // one kernel per (model, stencil) group, each on its own pair
-            // of counters
-            // of a launch: the first after k_batch_events in stream order,
-            // the others overlapping the one before
-            int32_t begin = 0;
-            bool first = true;
-            for (int g = 0; g < kGroups; ++g) {
-                const int32_t end = b->group_end[g];
-                if (end > begin) {
-                    const int grid = end - begin < b->grid ? end - begin : b->grid;
-                    int rc = batch_group_launch(g, pair, false, !first, grid, desc_t, tl_t,
-                                                begin, end, b->n_tissues, in_buf,
-                                                scratch + 2 + 2 * g, stream);
-                    if (rc) return rc;
-                    first = false;
+            if (li == 0 || by_group) {
+                const dim3 eb(32, 4);
+                k_batch_events<<<(unsigned)((b->n_tissues + 3) / 4), eb, 0, stream>>>(
+                    desc_t, b->n_tissues, offset + done, (int32_t)ks, in_buf);
+                FW_CHECK_LAUNCH("k_batch_events");
+            }
+            if (by_group) {
+                // each group on its own pair of counters, the first after
+                // k_batch_events in stream order, the others overlapping
+                // the one before
+                int32_t begin = 0;
+                bool first = true;
+                for (int g = 0; g < kGroups; ++g) {
+                    const int32_t end = b->group_end[g];
+                    if (end > begin) {
+                        const int n = end - begin < b->grid ? end - begin : b->grid;
+                        int rc = batch_group_launch(g, pair, false, !first, n, desc_t,
+                                                    tl_t, begin, end, b->n_tissues, in_buf,
+                                                    kRun, scratch + 2 + 2 * g, stream);
+                        if (rc) return rc;
+                        first = false;
+                    }
+                    begin = end;
                 }
-                begin = end;
+            } else {
+                k.in_buf = in_buf;
+                k.next_koff = offset + done + ks;
+                const int64_t more = left - ks, more_l = launches_left - 1;
+                k.next_ks = more_l > 0 ? (int32_t)std::min<int64_t>(
+                                             KMAX, (more + more_l - 1) / more_l) : 0;
+                (pair ? k_batch_all<true> : k_batch_all<false>)
+                    <<<grid, kTmaNT, kTmaSmem, stream>>>(k);
+                FW_CHECK_LAUNCH("k_batch_all");
             }
         } else {
             k_batch<<<b->grid, NT, kSmem, stream>>>(desc, tl, b->n_tiles,
