@@ -127,6 +127,12 @@ class Batch(ctypes.Structure):
                 ("reserved", _i32), ("group_end", _i32 * 6)]
 
 
+class Rows(ctypes.Structure):
+    _fields_ = [("src", _vp), ("dst", _vp), ("rows", _i64),
+                ("row_bytes", _i64), ("src_pitch", _i64),
+                ("dst_pitch", _i64)]
+
+
 class FwError(RuntimeError):
     """A non-OK status from libfwgpu."""
 
@@ -154,6 +160,8 @@ _SIGS = {
     "fw_ionic": ([_i32, _i32, _vp, _vp, _vp, _vp, _i64, _f64, _vp, _vp],
                  _i32),
     "fw_step": ([ctypes.POINTER(StepArgs), _i64, _i64, _vp], _i32),
+    "fw_nonmyo_differ": ([_vp, _vp, _vp, _i32, _i64, _vp, _vp], _i32),
+    "fw_copy_rows": ([_vp, _i32, _vp], _i32),
     "fw_node_list": ([_vp, _i64, _vp, _vp, _vp], _i32),
     "fw_pack_weights": ([_i32, _vp, _i64, _vp, _vp], _i32),
     "fw_ecg": ([_i32, _i32, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _i32, _f64,
@@ -169,7 +177,7 @@ _SIGS = {
 # symbol -> ctypes structure whose size must match the library's
 _STRUCTS = {0: StepArgs, 1: Stim, 2: AtTracker, 3: LatTracker,
             4: ProbeTracker, 5: Window, 6: Batch, 7: EcgTracker,
-            8: TipTracker, 9: Tip}
+            8: TipTracker, 9: Tip, 10: Rows}
 
 
 def load(path=None):

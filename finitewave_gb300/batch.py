@@ -32,9 +32,9 @@ class _Mirror:
     node-major packing) and the local activation tracker's flags -- with
     rows padded to a multiple of 16 nodes (the row pitch a tensor map
     needs).  The padding columns are non-myocytes holding zero in both
-    potential buffers.  The batch advances the copies; `sync_in` and
-    `sync_out` move the model's state between them and the model's own
-    arrays, and `swap` follows the model's u / u_new exchange."""
+    potential buffers.  The batch advances the copies; `copies_in` and
+    `copies_out` list the copies that move the model's state between them
+    and the model's own arrays, and `swap` follows the model's u / u_new exchange."""
 
     def __init__(self, m):
         ni, nj = m._shape()
@@ -74,14 +74,21 @@ class _Mirror:
                 and tracker.is_native(tr)
                 and getattr(tr, "_activated", None) is not None]
 
-    def sync_in(self):
-        m, nj = self.model, self.nj
+    def _rows(self, src, dst, nj_src, nj_dst):
+        """The copy of one array's rows between the model's layout (rows of
+        nj nodes) and the padded one (rows of `pitch`)."""
+        ni, b = self.u[0].shape[0], src.element_size()
+        return (src.data_ptr(), dst.data_ptr(), ni, self.nj * b, nj_src * b,
+                nj_dst * b)
+
+    def copies_in(self):
+        m, nj, P = self.model, self.nj, self.pitch
         ni = self.u[0].shape[0]
-        self.u[0][:, :nj].copy_(m._dev["u"])
-        self.u[1][:, :nj].copy_(m._dev["u_new"])
+        out = [self._rows(m._dev["u"], self.u[0], nj, P),
+               self._rows(m._dev["u_new"], self.u[1], nj, P)]
         for t, tb, name in zip(self.state, self.state_b, m._state_names):
-            t[:, :nj].copy_(m._dev[name])
-            tb[:, :nj].copy_(m._dev[name])
+            out.append(self._rows(m._dev[name], t, nj, P))
+            out.append(self._rows(m._dev[name], tb, nj, P))
         act = {}
         for f in self._lat_flags():
             old = self.act.get(f.data_ptr())
@@ -90,19 +97,20 @@ class _Mirror:
             else:
                 pad = torch.zeros((ni, self.pitch), dtype=torch.uint8,
                                   device=f.device)
-            pad[:, :nj].copy_(f.view(ni, nj))
+            out.append(self._rows(f, pad, nj, P))
             act[f.data_ptr()] = (f, pad)
         self.act = act
+        return out
 
-    def sync_out(self):
-        m, nj = self.model, self.nj
-        ni = self.u[0].shape[0]
-        m._dev["u"].copy_(self.u[0][:, :nj])
-        m._dev["u_new"].copy_(self.u[1][:, :nj])
+    def copies_out(self):
+        m, nj, P = self.model, self.nj, self.pitch
+        out = [self._rows(self.u[0], m._dev["u"], P, nj),
+               self._rows(self.u[1], m._dev["u_new"], P, nj)]
         for t, name in zip(self.state, m._state_names):
-            m._dev[name].copy_(t[:, :nj])
+            out.append(self._rows(t, m._dev[name], P, nj))
         for f, pad in self.act.values():
-            f.view(ni, nj).copy_(pad[:, :nj])
+            out.append(self._rows(pad, f, P, nj))
+        return out
 
     def swap(self):
         self.u.reverse()
@@ -125,6 +133,13 @@ class _Mirror:
             a.lat[k].activated = pad[1].data_ptr()
         a.pitch = self.pitch
         a.fused_variant = 0
+
+
+def _copy_rows(copies, stream):
+    """Run the copies (src, dst, rows, row bytes, source and destination
+    pitch in bytes), up to 64 a launch."""
+    arr = (_ffi.Rows * len(copies))(*copies)
+    _ffi.call("fw_copy_rows", arr, len(copies), stream)
 
 
 class TissueBatch:
@@ -253,22 +268,29 @@ class TissueBatch:
             if m.state_loader:
                 m.state_loader.load()
             m._nonmyo_equal = None
-            self._check(m)
         dev = self._device()
+        # one answer read back for all models
+        asked = [m for m in ms if getattr(m, "_differ", None) is not None]
+        for m in asked:
+            m._launch_nonmyo_check()
+        if asked:
+            for m, d in zip(asked, torch.cat([m._differ for m in asked]).tolist()):
+                m._read_nonmyo_check(d)
+        for m in ms:
+            self._check(m)
         remaining = [int(np.ceil((m.t_max - m.t) / m.dt)) for m in ms]
         active = [i for i in range(len(ms)) if remaining[i] > 0]
         stream = torch.cuda.current_stream(dev).cuda_stream
         tma = self.kernel in ("tma", "pairs")
         mirrors = [self._mirror(m) for m in ms] if tma else None
         if tma:
-            for mir in mirrors:
-                mir.sync_in()
+            _copy_rows([c for mir in mirrors for c in mir.copies_in()], stream)
         while active:
             limit = min(_MAX_SEGMENT, min(remaining[i] for i in active))
             if self.chunk:
                 limit = min(limit, int(self.chunk))
             n = min(ms[i]._segment_times(limit)[2] for i in active)
-            segs = [ms[i]._prepare_segment(n) for i in active]
+            segs = [ms[i]._prepare_segment(n, tune=False) for i in active]
             for i, seg in zip(active, segs):
                 if tma:
                     mirrors[i].apply(seg.args)
@@ -297,13 +319,13 @@ class TissueBatch:
                 remaining[i] -= n
                 host = tma and (m.command_sequence or m.state_saver)
                 if host:
-                    mirrors[i].sync_out()
+                    _copy_rows(mirrors[i].copies_out(), stream)
                 if m.command_sequence:
                     m.command_sequence.execute_next()
                 if m.state_saver:
                     m.state_saver.save()
                 if host:
-                    mirrors[i].sync_in()
+                    _copy_rows(mirrors[i].copies_in(), stream)
                 if m.check_termination():
                     if m.state_saver:
                         m.state_saver.save()
@@ -312,7 +334,6 @@ class TissueBatch:
                     still.append(i)
             active = still
         if tma:
-            for mir in mirrors:
-                mir.sync_out()
-        for m in ms:
-            m._check_status()
+            _copy_rows([c for mir in mirrors for c in mir.copies_out()], stream)
+        for m, st in zip(ms, torch.cat([m._status for m in ms]).tolist()):
+            m._check_status(st)

@@ -207,6 +207,7 @@ size_t fw_struct_size(int32_t which)
     case 7: return sizeof(fw_ecg_tracker);
     case 8: return sizeof(fw_tip_tracker);
     case 9: return sizeof(fw_tip);
+    case 10: return sizeof(fw_rows);
     }
     return 0;
 }
@@ -284,6 +285,17 @@ int fw_ionic(int32_t model, int32_t precision, void *u_new, const void *u,
         }
     return fw::ionic(model, precision, u_new, u, state, idx, n_idx, dt, params,
                      (cudaStream_t)stream);
+}
+
+int fw_nonmyo_differ(const int8_t *myo, const void *u0, const void *u1,
+                     int32_t precision, int64_t n, int32_t *flag, void *stream)
+{
+    return fw::nonmyo_differ(myo, u0, u1, precision, n, flag, (cudaStream_t)stream);
+}
+
+int fw_copy_rows(const fw_rows *copies, int32_t n, void *stream)
+{
+    return fw::copy_rows(copies, n, (cudaStream_t)stream);
 }
 
 int fw_node_list(const int8_t *myo, int64_t n, int32_t *list, int32_t *scratch,

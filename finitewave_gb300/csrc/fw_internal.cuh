@@ -184,6 +184,9 @@ int ecg(int32_t stencil, int32_t precision, const void *u, const void *w,
         cudaStream_t stream);
 int step_fused(const fw_step_args *a, int64_t n_begin, int64_t n_steps,
                cudaStream_t stream);
+int nonmyo_differ(const int8_t *myo, const void *u0, const void *u1,
+                  int32_t precision, int64_t n, int32_t *flag, cudaStream_t stream);
+int copy_rows(const fw_rows *copies, int32_t n, cudaStream_t stream);
 int node_list(const int8_t *myo, int64_t n, int32_t *list, int32_t *scratch,
               cudaStream_t stream);
 int pack_weights(int32_t stencil, const float *w, int64_t n, float *out,

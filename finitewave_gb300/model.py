@@ -34,6 +34,8 @@ _MAX_SEGMENT = 1 << 20
 
 
 def _np_name(npfloat):
+    if type(npfloat) is str and npfloat in _NP:
+        return npfloat
     name = np.dtype(npfloat).name
     if name not in _NP:
         raise ValueError(f"npfloat must be float64 or float32, got {npfloat}")
@@ -241,6 +243,7 @@ class CardiacModel:
         self.t = 0
         self._t_hist = []
         self._status = torch.zeros(1, dtype=torch.int32, device=dev)
+        self._differ = torch.zeros(1, dtype=torch.int32, device=dev)
         self.compute_weights()
         self.diffusion_kernel = self.stencil.select_diffusion_kernel()
         if self.stim_sequence:
@@ -569,10 +572,23 @@ class CardiacModel:
                     for t in trs) > 1):
             return False
         if getattr(self, "_nonmyo_equal", None) is None:
-            off = self._myo_d == 0
-            self._nonmyo_equal = bool(torch.equal(self._dev["u"][off],
-                                                  self._dev["u_new"][off]))
+            self._launch_nonmyo_check()
+            self._read_nonmyo_check(int(self._differ.item()))
         return self._nonmyo_equal
+
+    def _launch_nonmyo_check(self):
+        """Ask the device whether u and u_new differ at a non-myocyte; the
+        answer lands in the flag `_differ`."""
+        u = self._dev["u"]
+        _ffi.call("fw_nonmyo_differ", self._myo_d.data_ptr(), u.data_ptr(),
+                  self._dev["u_new"].data_ptr(), self._precision(), u.numel(),
+                  self._differ.data_ptr(),
+                  torch.cuda.current_stream().cuda_stream)
+
+    def _read_nonmyo_check(self, differ):
+        self._nonmyo_equal = not differ
+        if differ:
+            self._differ.zero_()
 
     def _form(self):
         if self.form == "plain":
@@ -627,9 +643,10 @@ class CardiacModel:
         self._finish_segment(seg)
         return seg.n_seg
 
-    def _bare_args(self):
+    def _bare_args(self, tune=True):
         """fw_step_args with the model's arrays, parameters and kernel
-        choice, and no stimuli or trackers."""
+        choice (none where the caller makes its own: tune=False), and no
+        stimuli or trackers."""
         a = _ffi.StepArgs()
         a.model = self._model_id
         a.stencil = getattr(self, "_step_stencil", self.stencil.kind)
@@ -669,7 +686,7 @@ class CardiacModel:
         if a.fused_variant == 5 and a.form == _ffi.FORM_FUSED:
             self._fly_args(a)
         if (a.form == _ffi.FORM_FUSED and not a.fused_k and
-                not a.fused_variant and self.autotune):
+                not a.fused_variant and self.autotune and tune):
             from . import autotune
             a.fused_variant, a.fused_k = autotune.choose(self)
         self._fused_choice = (a.fused_variant, a.fused_k) \
@@ -699,12 +716,12 @@ class CardiacModel:
         a.fly_cond = float(tissue.conductivity)
         a.fly_scale = float(self.D_model) * float(self.dt) / float(self.dr) ** 2
 
-    def _prepare_segment(self, limit, skip_stims=False):
+    def _prepare_segment(self, limit, skip_stims=False, tune=True):
         """The fw_step_args of the next segment of at most `limit` steps
         (stimulus and tracker windows in global step indices).  Stimuli and
         trackers that run on the host are left out, and so are all stimuli
         with skip_stims (a host step that has applied them already)."""
-        a = self._bare_args()
+        a = self._bare_args(tune)
         ts, t_end, n_seg = self._segment_times(limit)
         n0 = int(self.step)
         self._t_hist.append(ts)

@@ -420,6 +420,24 @@ FW_API int fw_ionic(int32_t model, int32_t precision, void *u_new, const void *u
              void *const *state, const int64_t *idx, int64_t n_idx,
              double dt, const double *params, void *stream);
 
+/* Sets *flag (device int32, left alone otherwise) when the two potential
+ * buffers u0 and u1 (n values, by precision) differ at a node of myo == 0:
+ * the fused form needs them equal there. */
+FW_API int fw_nonmyo_differ(const int8_t *myo, const void *u0, const void *u1,
+             int32_t precision, int64_t n, int32_t *flag, void *stream);
+
+/* One two-dimensional copy between device arrays: `rows` rows of
+ * `row_bytes` bytes, their starts src_pitch / dst_pitch bytes apart. */
+typedef struct fw_rows {
+    const void *src;
+    void *dst;
+    int64_t rows, row_bytes, src_pitch, dst_pitch;
+} fw_rows;
+
+/* n such copies, any number per launch up to 64 (the tissues of a batch move
+ * in and out of their row-padded copies).  The arrays must not overlap. */
+FW_API int fw_copy_rows(const fw_rows *copies, int32_t n, void *stream);
+
 /* fw_step_args.node_list of a grid: the n < 2^31 nodes with those of
  * myo != 0 first, each part in ascending order, written to list (n).
  * scratch: device int32, n / 4096 + 2 values. */
