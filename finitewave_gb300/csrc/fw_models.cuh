@@ -164,10 +164,11 @@ struct ModelAP {
             const T cub = fmaf(ua1, u, a) * u;
             return fmaf(dt, fmaf(-k, cub, -(u * v)), un);
         } else {
-            v += (-dt) * (eap + (mu_1 * v) / (mu_2 + u)) *
-                 (v + k * u * (u - a - (T)1.));
+            // (-k) u is -(k u): one product for both equations
+            const T ku = k * u, ua = u - a;
+            v += (-dt) * (eap + (mu_1 * v) / (mu_2 + u)) * (v + ku * (ua - (T)1.));
             x.v = v;
-            return un + dt * ((-k) * u * (u - a) * (u - (T)1.) - u * v);
+            return un + dt * ((-ku) * ua * (u - (T)1.) - u * v);
         }
     }
     // The float32 update of the fused and batched kernels: update<float>'s

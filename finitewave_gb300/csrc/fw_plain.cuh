@@ -10,9 +10,10 @@
 //   2. k_step      all nodes: trackers read u_cur (after stimuli, before the
 //                  update, as tracker_next does after the kernels but before
 //                  the swap); myocytes get u_nxt = diffusion + ionic
-//   3. k_probe     when a probe tracker is active at n: u_cur and the state
-//                  variables (already advanced, as the reference's trackers
-//                  see them)
+//   3. k_probe     when a probe tracker of state variables is active at n:
+//                  u_cur and the state (already advanced, as the reference's
+//                  trackers see them); probes of u alone are sampled inside
+//                  k_step
 //   the caller's buffers then swap roles.
 #pragma once
 
@@ -80,6 +81,13 @@ struct LatK {
     int32_t cap;
 };
 
+// A probe tracker's sample of the potential: out[c] = u[cells[c]].
+struct UProbe {
+    const int64_t *cells;
+    double *out;
+    int32_t n_cells;
+};
+
 template <class M, class T>
 struct StepK {
     const int8_t *myo;
@@ -103,6 +111,9 @@ struct StepK {
     AtK<T> at[FW_MAX_AT];
     LatK<T> lat[FW_MAX_LAT];
     int32_t *status;
+    // probes of the potential alone, sampled by the launch's last CTA
+    int32_t n_up;
+    UProbe up[FW_MAX_PROBE];
 };
 
 // isfinite on the bits: the comparison would take a turn of the float64 pipe
@@ -112,12 +123,23 @@ __device__ __forceinline__ bool finite_bits(double x)
 }
 __device__ __forceinline__ bool finite_bits(float x) { return isfinite(x); }
 
+// True wherever x > y: the same comparison on the bits as integers, which
+// most nodes fail, so that the float64 pipe is asked only about the others.
+__device__ __forceinline__ bool maybe_above(double x, double y)
+{
+    long long a = __double_as_longlong(x), b = __double_as_longlong(y);
+    a ^= (a >> 63) & 0x7fffffffffffffffll;
+    b ^= (b >> 63) & 0x7fffffffffffffffll;
+    return a > b;
+}
+__device__ __forceinline__ bool maybe_above(float, float) { return true; }
+
 template <class M, class T>
 __device__ __forceinline__ void track(const StepK<M, T> &k, int64_t p, T uc)
 {
     for (int a = 0; a < k.n_at; ++a) {
         // (act_t < 0) & (u > threshold)  (activation_time_2d_tracker.py:61-63)
-        if (uc > k.at[a].thr && k.at[a].act[p] < 0)
+        if (maybe_above(uc, k.at[a].thr) && uc > k.at[a].thr && k.at[a].act[p] < 0)
             k.at[a].act[p] = (int32_t)k.step;
     }
     for (int l = 0; l < k.n_lat; ++l) {
@@ -195,8 +217,26 @@ __global__ void __launch_bounds__(step_threads<T>(), (MinBlocks<M, T>::value))
     const Params<T, M::NP + M::ND> P = load_params<T, M::NP + M::ND>(k.params);
     const T dt = k.dt;
     const int64_t n = LIST ? (int64_t)k.n_run : k.n;
+    // Steps of one call follow one another with programmatic serialisation:
+    // the next one's CTAs take their places, read their parameters and wait
+    // here while this one's last CTAs run.  A listed float64 step lets them
+    // come only when a CTA is done: placed earlier, in the slots that this
+    // step's CTAs leave, they would not spread evenly over the SMs, whose
+    // float64 pipes set the time (TP06 192 x 190: 68 against 61 us a step).
+    // One step of Courtemanche float32 511 x 387 takes 6.6 us so, 8.4 without;
+    // of Aliev-Panfilov float32 256 x 240 x 60 59 against 62.
+    constexpr bool kLate = LIST && sizeof(T) == 8;
+    if constexpr (!kLate) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (k.n_up && blockIdx.x == gridDim.x - 1) {
+        for (int a = 0; a < k.n_up; ++a)
+            for (int c = threadIdx.x; c < k.up[a].n_cells; c += blockDim.x)
+                k.up[a].out[c] = (double)k.u[k.up[a].cells[c]];
+        return;
+    }
+    const int64_t stride = (int64_t)(gridDim.x - (k.n_up ? 1 : 0)) * blockDim.x;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
-         t += (int64_t)gridDim.x * blockDim.x) {
+         t += stride) {
         const int64_t p = LIST ? (int64_t)k.list[t] : t;
         T uc = k.u[p];
         if (k.n_at | k.n_lat) track(k, p, uc);
@@ -217,6 +257,7 @@ __global__ void __launch_bounds__(step_threads<T>(), (MinBlocks<M, T>::value))
         k.un[p] = un;
         if (!finite_bits(un) && k.status) atomicOr(k.status, FW_DEV_NONFINITE);
     }
+    if constexpr (kLate) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 struct ProbeOne {
@@ -575,6 +616,13 @@ int run_plain(const fw_step_args *a, int64_t n_begin, int64_t n_steps,
     k.n_myo = (int32_t)a->n_list_myo;
     const int blocks_all = grid_for(g.n, threads, step_blocks<M, T>());
     const int blocks_myo = grid_for(a->n_list_myo, threads, step_blocks<M, T>());
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(threads);
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
     for (int64_t s = 0; s < n_steps; ++s) {
         const int64_t n = n_begin + s;
         T *cur = (T *)a->u[s & 1];
@@ -602,31 +650,39 @@ int run_plain(const fw_step_args *a, int64_t n_begin, int64_t n_steps,
                                         L.cross_steps, L.cross_count,
                                         L.capacity};
             }
-        // the trackers also watch the nodes that do not step
-        const bool all = k.n_at || k.n_lat || !listed;
-        k.n_run = all ? (int32_t)(listed ? g.n : 0) : k.n_myo;
-        bool launched = false;
-        if constexpr (UseList<M, T>::value) {
-            if (listed && k.n_run > 0)
-                k_step<M, ST, T, true><<<all ? blocks_all : blocks_myo, threads, 0,
-                                         stream>>>(k);
-            launched = listed;
-        }
-        if (!launched)
-            k_step<M, ST, T, false><<<blocks_all, threads, 0, stream>>>(k);
-        FW_CHECK_LAUNCH("k_step");
+        // probes of the potential alone ride on the step; those of the state,
+        // which the step advances, follow it
         pk.n = 0;
+        k.n_up = 0;
         for (int i = 0; i < a->n_probe; ++i) {
             const fw_probe_tracker &P = a->probe[i];
             if (!in_window(P.win, n)) continue;
+            const int64_t sample = P.sample_offset + (n - P.win.first) / P.win.stride;
+            if (P.n_vars == 1 && P.var_ids[0] == 0 && sample < P.capacity) {
+                k.up[k.n_up++] = UProbe{P.cells, P.out + sample * P.n_cells, P.n_cells};
+                continue;
+            }
             ProbeOne &o = pk.pr[pk.n++];
             o.cells = P.cells;
             o.out = P.out;
-            o.sample = P.sample_offset + (n - P.win.first) / P.win.stride;
+            o.sample = sample;
             o.capacity = P.capacity;
             o.n_cells = P.n_cells;
             o.n_vars = P.n_vars;
             for (int v = 0; v < FW_MAX_PROBE_VARS; ++v) o.var_ids[v] = P.var_ids[v];
+        }
+        // the trackers also watch the nodes that do not step
+        const bool all = k.n_at || k.n_lat || !listed;
+        k.n_run = all ? (int32_t)(listed ? g.n : 0) : k.n_myo;
+        attr.val.programmaticStreamSerializationAllowed = s > 0;
+        cfg.gridDim = dim3((unsigned)((all ? blocks_all : blocks_myo) + (k.n_up ? 1 : 0)));
+        auto kern = k_step<M, ST, T, false>;
+        if constexpr (UseList<M, T>::value) {
+            if (listed) kern = k_step<M, ST, T, true>;
+        }
+        if (!listed || k.n_run > 0 || k.n_up) {
+            FW_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, k));
+            FW_CHECK_LAUNCH("k_step");
         }
         if (pk.n) {
             pk.u = cur;
