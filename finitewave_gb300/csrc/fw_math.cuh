@@ -287,17 +287,6 @@ __device__ __forceinline__ float ex2(float x)
     return y;
 }
 __device__ __forceinline__ float ex(float x) { return ex2(x * (float)kLog2e); }
-__device__ __forceinline__ float ex_limited(float x) { return ex(x); }
-// with the rounding of x log2(e) put back
-__device__ __forceinline__ float ex_near(float x)
-{
-    const float t = x * (float)kLog2e;
-    const float lo = fmaf(x, (float)(kLog2e - (double)(float)kLog2e),
-                          fmaf(x, (float)kLog2e, -t));
-    const float e = ex2(t);
-    return fmaf(e, lo * 0.693147181f, e);
-}
-__device__ __forceinline__ double ex_near(double x) { return ex(x); }
 __device__ __forceinline__ float lg(float x) { return __logf(x); }
 __device__ __forceinline__ float rcp(float d)
 {

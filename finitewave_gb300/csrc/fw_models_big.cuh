@@ -5,8 +5,8 @@
 // currents and the concentration rates; the ion-concentration state (TP06:
 // Ca_i, Ca_SR, Ca_ss, Na_i, K_i; Courtemanche: Na_i, K_i, Ca_i, Ca_up,
 // Ca_rel; Luo-Rudy 1991: Ca_i) takes 8 bytes per node in both forms.  Under
-// FW_F64 every quantity is float64.  Each update comes twice: in a form with
-// few divisions and exponentials (fw_math.cuh) for the potentials of a
+// FW_F64 every quantity is float64, and the update comes twice: in a form
+// with few divisions and exponentials (fw_math.cuh) for the potentials of a
 // simulation, and in the reference's evaluation order, with CUDA's
 // exp/log/sqrt/pow, for any other.  Under FW_F32 everything is computed in float32 from the
 // concentrations rounded to float, and the accumulation `c += dt * rate`
@@ -848,15 +848,21 @@ struct ModelCRN {
     __device__ static __forceinline__ T update(T u, T un, St<T> &x,
                                                const Params<T, NP + ND> &P, T dt)
     {
-        if (in_range(u)) return update_in_range<T>(u, un, x, P, dt);
-        return update_any<T>(u, un, x, P, dt);
+        if constexpr (sizeof(T) == 4) {
+            // float32 keeps the reference's order and with it the bits of its
+            // results: the rates of h jump by a quarter at u = -40, so a node
+            // that meets the branch a step earlier for another rounding
+            // differs by 1e-3 there
+            return update_ref<T>(u, un, x, P, dt);
+        } else {
+            if (in_range(u)) return update_in_range<T>(u, un, x, P, dt);
+            return update_any<T>(u, un, x, P, dt);
+        }
     }
     __device__ static __forceinline__ bool in_range(double u) { return fabs(u) < 300.0; }
-    __device__ static __forceinline__ bool in_range(float u) { return fabsf(u) < 130.f; }
 
-    // As ModelTP06::update_in_range: one quotient per rate.  float64
-    // 192 x 190 nodes: 65 against 180 us a step; float32 511 x 387 nodes:
-    // 8.4 against 10.4.
+    // As ModelTP06::update_in_range (float64 only): one quotient per rate.
+    // 192 x 190 nodes: 65 against 180 us a step.
     template <class T>
     __device__ static __forceinline__ T update_in_range(T u, T un, St<T> &x,
                                                         const Params<T, NP + ND> &P,
@@ -878,9 +884,7 @@ struct ModelCRN {
         {
             const T z = (T)(-0.1) * (u + (T)47.13);
             T am = (T)3.2 * x_over_expm1(z, ex(z));
-            if constexpr (sizeof(T) == 8) {
-                if (u == (T)(-47.13)) am = (T)3.2;
-            }
+            if (u == (T)(-47.13)) am = (T)3.2;
             const T sm = am + (T)0.08 * FW_EX(u, -1 / 11.0);
             x.m = gate_fast(x.m, div_near(am, sm), ndt, sm);
             T h_inf = (T)0, j_inf = (T)0, rate_h, rate_j;
@@ -1019,8 +1023,8 @@ struct ModelCRN {
                           inaca + ibna + ibca);
     }
 
-    // The update in the reference's order, for potentials outside the range
-    // above.
+    // The update in the reference's order: float32, and float64 potentials
+    // outside the range above.
     // (Copies go into the call, so that x and P keep to registers elsewhere.)
     template <class T>
     __device__ static __forceinline__ T update_any(T u, T un, St<T> &x,
@@ -1320,21 +1324,25 @@ struct ModelLR91 {
     __device__ static __forceinline__ T update(T u, T un, St<T> &x,
                                                const Params<T, NP + ND> &P, T dt)
     {
-        if (in_range(u, u - P.v[d_ek1])) return update_in_range<T>(u, un, x, P, dt);
-        return update_any<T>(u, un, x, P, dt);
+        if constexpr (sizeof(T) == 4) {
+            // float32 keeps the reference's order and with it the bits of its
+            // results: the rates of h jump by a quarter at u = -40, so a node
+            // that meets the branch a step earlier for another rounding
+            // differs by 1e-3 there
+            return update_ref<T>(u, un, x, P, dt);
+        } else {
+            if (in_range(u, u - P.v[d_ek1])) return update_in_range<T>(u, un, x, P, dt);
+            return update_any<T>(u, un, x, P, dt);
+        }
     }
     __device__ static __forceinline__ bool in_range(double u, double x)
     {
         return fabs(u) < 300.0 && x > -400.0 && x < 1000.0;
     }
-    __device__ static __forceinline__ bool in_range(float u, float x)
-    {
-        return fabsf(u) < 130.f && x > -100.f && x < 230.f;
-    }
 
     // As ModelTP06::update_in_range; var + dt (inf - var) / tau with
     // tau = 1 / (a + b), inf = a / (a + b) is var + dt (a (1 - var) - b var).
-    // float64 192 x 190 nodes: 33 against 75 us a step.
+    // 192 x 190 nodes: 33 against 75 us a step (float64 only).
     template <class T>
     __device__ static __forceinline__ T update_in_range(T u, T un, St<T> &x,
                                                         const Params<T, NP + ND> &P,
@@ -1363,10 +1371,8 @@ struct ModelLR91 {
                           (u + (T)37.78) * rcp(c1 + FW_EX(u + (T)79.23, 0.311));
             }
             const T z = (T)(-0.1) * (u + (T)47.13);
-            const T alpha_m = (T)3.2 * x_over_expm1(z, ex_near(z));
-            T beta_m;
-            if constexpr (sizeof(T) == 8) beta_m = (T)0.08 * FW_EX(u, -1 / 11.0);
-            else beta_m = (T)0.08 * ex_near(u * (T)(-1 / 11.0));
+            const T alpha_m = (T)3.2 * x_over_expm1(z, ex(z));
+            const T beta_m = (T)0.08 * FW_EX(u, -1 / 11.0);
             x.m = gate(x.m, alpha_m, beta_m);
             x.h = gate(x.h, alpha_h, beta_h);
             x.j = gate(x.j, alpha_J, beta_J);
@@ -1415,8 +1421,8 @@ struct ModelLR91 {
         return un - dt * (ina + isi + (ik1 + ikp + ib) + ik);
     }
 
-    // The update in the reference's order, for potentials outside the range
-    // above.
+    // The update in the reference's order: float32, and float64 potentials
+    // outside the range above.
     // (Copies go into the call, so that x and P keep to registers elsewhere.)
     template <class T>
     __device__ static __forceinline__ T update_any(T u, T un, St<T> &x,
