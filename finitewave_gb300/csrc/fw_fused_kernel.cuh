@@ -222,10 +222,9 @@ __device__ __forceinline__ float2 stencil_fma2(float2 wcen, float2 c, const floa
     return un;
 }
 
-// The ionic update of the fused and batched kernels: a model with a
-// two-node form (M::update_pair) uses its explicitly rounded float32
-// update (M::update_fused), which the pair form reproduces per node;
-// otherwise update<float>, once per node.
+// The ionic update of the fused and batched kernels (M::update_fused), and
+// its two-node form, which gives each node the same bits: M::update_pair
+// where the model has one, else update_fused once per node.
 template <class M, class = void>
 struct has_pair_form : std::false_type {};
 template <class M>
@@ -236,10 +235,7 @@ __device__ __forceinline__ float fused_update(float u, float un,
                                               typename M::template St<float> &x,
                                               const Params<float, M::NP> &P, float dt)
 {
-    if constexpr (has_pair_form<M>::value)
-        return M::update_fused(u, un, x, P, dt);
-    else
-        return M::template update<float>(u, un, x, P, dt);
+    return M::update_fused(u, un, x, P, dt);
 }
 
 template <class M>
@@ -252,8 +248,8 @@ __device__ __forceinline__ float2 fused_update_pair(float2 u, float2 un,
     if constexpr (has_pair_form<M>::value) {
         return M::update_pair(u, un, x0, x1, P, dt);
     } else {
-        const float a = M::template update<float>(u.x, un.x, x0, P, dt);
-        const float b = M::template update<float>(u.y, un.y, x1, P, dt);
+        const float a = M::update_fused(u.x, un.x, x0, P, dt);
+        const float b = M::update_fused(u.y, un.y, x1, P, dt);
         return make_float2(a, b);
     }
 }

@@ -211,6 +211,17 @@ struct ModelAP {
     }
 };
 
+// The fused kernels' float32 updates of the next models (update_fused): the
+// same expressions, each quotient by a parameter taken as a product with the
+// parameter's reciprocal, which the compiler forms once a tile.  A quotient
+// under --prec-div=false is that reciprocal and product, bit for bit while
+// the divisor is within 2^-126 .. 2^126, but costs six instructions every
+// time; the product stays out of any fused multiply-add, as the quotient did.
+__device__ __forceinline__ float over(float a, float b)
+{
+    return a * dm::rcp(b);
+}
+
 // Mitchell-Schaeffer.  params: tau_close, tau_open, tau_in, tau_out, u_gate
 // (mitchell_schaeffer_2d.py:57-61).  calc_h, calc_J_in, calc_J_out,
 // ionic_kernel_2d (:102-217).  u**2 is u*u as numba compiles it.
@@ -254,6 +265,21 @@ struct ModelMS {
         T C = (u * u) * ((T)1 - u);
         T J_in = h * C / tau_in;
         T J_out = -u / tau_out;
+        return un + dt * (J_in + J_out);
+    }
+    __device__ static __forceinline__ float update_fused(float u, float un,
+                                                         St<float> &x,
+                                                         const Params<float, NP> &P,
+                                                         float dt)
+    {
+        const float tau_close = P.v[0], tau_open = P.v[1], tau_in = P.v[2],
+                    tau_out = P.v[3], u_gate = P.v[4];
+        float h = x.h;
+        h += (u < u_gate) ? over(dt * (1.f - h), tau_open) : over(dt * (-h), tau_close);
+        x.h = h;
+        const float C = (u * u) * (1.f - u);
+        const float J_in = over(h * C, tau_in);
+        const float J_out = over(-u, tau_out);
         return un + dt * (J_in + J_out);
     }
 };
@@ -310,6 +336,27 @@ struct ModelFK {
         T J_si = (-v) * (one + fw_tanh(k * (u - uc_si))) / ((T)2 * tau_si);
         return un + dt * (-J_fi - J_so - J_si);
     }
+    __device__ static __forceinline__ float update_fused(float u, float un,
+                                                         St<float> &x,
+                                                         const Params<float, NP> &P,
+                                                         float dt)
+    {
+        const float tau_d = P.v[0], tau_o = P.v[1], tau_r = P.v[2], tau_si = P.v[3],
+                    tau_v_m = P.v[4], tau_v_p = P.v[5], tau_w_m = P.v[6],
+                    tau_w_p = P.v[7], k = P.v[8], u_c = P.v[9], uc_si = P.v[10];
+        const float H1 = (u_c - u) >= 0 ? 1.f : 0.f;
+        const float H2 = (u - u_c) >= 0 ? 1.f : 0.f;
+        const float v = x.v + dt * (over(H1 * (1.f - x.v), tau_v_m) -
+                                    over(H2 * x.v, tau_v_p));
+        const float w = x.w + dt * (over(H1 * (1.f - x.w), tau_w_m) -
+                                    over(H2 * x.w, tau_w_p));
+        x.v = v;
+        x.w = w;
+        const float J_fi = over(-(v * H2 * (1.f - u) * (u - u_c)), tau_d);
+        const float J_so = over(u * H1, tau_o) + over(H2, tau_r);
+        const float J_si = over((-v) * (1.f + fw_tanh(k * (u - uc_si))), 2.f * tau_si);
+        return un + dt * (-J_fi - J_so - J_si);
+    }
 };
 
 // Barkley.  params: a, b, eap (barkley_2d.py:69-71, ionic_kernel_2d
@@ -351,6 +398,17 @@ struct ModelBK {
         v += dt * (u - v);
         x.v = v;
         return un + dt * (u * ((T)1 - u) * (u - (v + b) / a)) / eap;
+    }
+    __device__ static __forceinline__ float update_fused(float u, float un,
+                                                         St<float> &x,
+                                                         const Params<float, NP> &P,
+                                                         float dt)
+    {
+        const float a = P.v[0], b = P.v[1], eap = P.v[2];
+        float v = x.v;
+        v += dt * (u - v);
+        x.v = v;
+        return un + over(dt * (u * (1.f - u) * (u - over(v + b, a))), eap);
     }
 };
 
