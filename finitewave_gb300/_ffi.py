@@ -118,7 +118,8 @@ class StepArgs(ctypes.Structure):
                 ("fibers_f32", _vp), ("fly_D_al", _f64), ("fly_D_ac", _f64),
                 ("fly_cond", _f64), ("fly_scale", _f64),
                 ("weight_rows", _vp), ("weight_row_index", _vp),
-                ("node_list", _vp), ("n_list_myo", _i64)]
+                ("node_list", _vp), ("n_list_myo", _i64),
+                ("weight_centre", _vp)]
 
 
 class Batch(ctypes.Structure):
@@ -162,6 +163,7 @@ _SIGS = {
     "fw_step": ([ctypes.POINTER(StepArgs), _i64, _i64, _vp], _i32),
     "fw_nonmyo_differ": ([_vp, _vp, _vp, _i32, _i64, _vp, _vp], _i32),
     "fw_copy_rows": ([_vp, _i32, _vp], _i32),
+    "fw_pack_rows": ([_i32, _vp, _i64, _i64, _i64, _vp, _vp, _vp], _i32),
     "fw_node_list": ([_vp, _i64, _vp, _vp, _vp], _i32),
     "fw_pack_weights": ([_i32, _vp, _i64, _vp, _vp], _i32),
     "fw_ecg": ([_i32, _i32, _vp, _vp, _vp, _i64, _i64, _i64, _vp, _i32, _f64,

@@ -28,8 +28,9 @@ from . import _ffi
 _lock = threading.Lock()
 _memo = {}
 
-# (fused_variant, fused_k) candidates; variants 3 and 4 only where the TMA
-# kernels can run (packed weights, nj % 16 == 0).  Variants 5, 6 and 7 are
+# (fused_variant, fused_k) candidates; variants 3 and 4 where the TMA kernels
+# can run (packed weights; rows of a multiple of 16 nodes, or padded copies of
+# the arrays).  Variants 5, 6 and 7 are
 # not candidates: each was measured slower than variant 3 on the 4096^2
 # Aliev-Panfilov workload (weights formed on chip, two-wide float32
 # instructions, the row-marching wavefront) and is kept as an explicit
@@ -71,8 +72,11 @@ def key(model):
         n *= s
     dev = model._device()
     name = torch.cuda.get_device_name(dev)
-    return "|".join([name, type(model).__name__, str(model.stencil.kind),
-                     "%dD" % len(shape), "2^%d" % int(math.log2(max(n, 1)))])
+    parts = [name, type(model).__name__, str(model.stencil.kind),
+             "%dD" % len(shape), "2^%d" % int(math.log2(max(n, 1)))]
+    if len(shape) == 2 and shape[1] % 16:
+        parts.append("ragged")   # the TMA kernels run on padded copies
+    return "|".join(parts)
 
 
 def _time_candidate(model, args, variant, k, steps, stream, reps=3):
@@ -125,10 +129,52 @@ def tune(model, steps=96):
                                                       stream)
         except _ffi.FwError:
             continue
+    # rows that are no multiple of 16 nodes: the TMA kernels on row-padded
+    # copies of the arrays, the copies in and out counted once in `steps`
+    # steps (777 x 1011 nodes: 25 us; Aliev-Panfilov 2500 x 2501 takes 28.8 us
+    # a step so, 37.5 on its own arrays, 500 x 501 2.8 against 2.1)
+    flat = min(times, key=times.get)
+    cost = dict(times)
+    if model._shape()[1] % 16 and model._pad_ok():
+        mir = model._padded()
+        copies = _time_copies(mir, stream)
+        mir.apply(a)
+        for v, k in _TMA:
+            try:
+                t = _time_candidate(model, a, v, k, steps, stream)
+            except _ffi.FwError:
+                continue
+            times["%d/%d" % (v, k)] = t
+            cost["%d/%d" % (v, k)] = t + copies
     del keep
-    best = min(times, key=times.get)
+    best = min(cost, key=cost.get)
     v, k = (int(x) for x in best.split("/"))
-    return {"variant": v, "k": k, "ms": times, "steps": steps}
+    fv, fk = (int(x) for x in flat.split("/"))
+    return {"variant": v, "k": k, "flat": [fv, fk], "ms": times, "steps": steps}
+
+
+def _time_copies(mir, stream, reps=3):
+    """ms of moving a model's state into its padded copies and, unchanged,
+    out again."""
+    best = float("inf")
+    for _ in range(reps):
+        e0 = torch.cuda.Event(enable_timing=True)
+        e1 = torch.cuda.Event(enable_timing=True)
+        e0.record(stream)
+        mir.run_copies(mir.copies_in(), stream.cuda_stream)
+        mir.run_copies(mir.copies_out(), stream.cuda_stream)
+        e1.record(stream)
+        e1.synchronize()
+        best = min(best, e0.elapsed_time(e1))
+    return best
+
+
+def choose_flat(model):
+    """The fastest candidate on the model's own arrays (rows of any length)."""
+    choose(model)
+    with _lock:
+        r = _memo[key(model)]
+    return tuple(r.get("flat") or (r["variant"], r["k"]))
 
 
 def choose(model):

@@ -28,13 +28,12 @@ _BATCH_MODELS = (_ffi.MODEL_AP, _ffi.MODEL_MS, _ffi.MODEL_FK)
 class _Mirror:
     """Copies of one model's arrays that the TMA form of the batched kernel
     reads through tensor maps -- the two potential buffers, the two buffers
-    of each state variable, the myocyte flags, the weights (plus their
-    node-major packing) and the local activation tracker's flags -- with
-    rows padded to a multiple of 16 nodes (the row pitch a tensor map
-    needs).  The padding columns are non-myocytes holding zero in both
-    potential buffers.  The batch advances the copies; `copies_in` and
-    `copies_out` list the copies that move the model's state between them
-    and the model's own arrays, and `swap` follows the model's u / u_new exchange."""
+    of each state variable, the myocyte flags, the packed weights and their
+    centre plane and the local activation tracker's flags -- with rows
+    padded to a multiple of 16 nodes (the row pitch a tensor map needs).
+    The batch advances the copies; `copies_in` and `copies_out` list the
+    copies that move the model's state between them and the model's own
+    arrays, and `swap` follows the model's u / u_new exchange."""
 
     def __init__(self, m):
         ni, nj = m._shape()
@@ -43,22 +42,22 @@ class _Mirror:
         self.weights_src = m.weights
         dev = m._device()
         f32 = torch.float32
-        nw = m.weights.shape[0]
-        self.w = torch.zeros((nw, ni, self.pitch), dtype=f32, device=dev)
-        self.w[:, :, :nj] = m.weights.view(nw, ni, nj)
         nwo = 4 if m.stencil.kind == _ffi.ISO5 else 8
         self.wpack = torch.empty(ni * self.pitch * nwo, dtype=f32, device=dev)
-        _ffi.call("fw_pack_weights", m.stencil.kind, self.w.data_ptr(),
-                  ni * self.pitch, self.wpack.data_ptr(),
-                  torch.cuda.current_stream(dev).cuda_stream)
-        self.myo = torch.zeros((ni, self.pitch), dtype=torch.int8, device=dev)
-        self.myo[:, :nj] = m._myo_d
-        self.u = [torch.zeros((ni, self.pitch), dtype=f32, device=dev)
-                  for _ in range(2)]
-        self.state = [torch.zeros((ni, self.pitch), dtype=f32, device=dev)
-                      for _ in m._state_names]
-        self.state_b = [torch.zeros((ni, self.pitch), dtype=f32, device=dev)
-                        for _ in m._state_names]
+        self.centre = torch.empty((ni, self.pitch), dtype=f32, device=dev)
+        stream = torch.cuda.current_stream(dev).cuda_stream
+        _ffi.call("fw_pack_rows", m.stencil.kind, m.weights.data_ptr(), ni, nj,
+                  self.pitch, self.wpack.data_ptr(), self.centre.data_ptr(),
+                  stream)
+        # the tensor maps end at column nj - 1: the padding is never read,
+        # except the pair view's weights, which are zero there
+        self.myo, *pots = (torch.empty((ni, self.pitch), dtype=t, device=dev)
+                           for t in [torch.int8] + [f32] * (2 + 2 * len(m._state_names)))
+        _copy_rows([(m._myo_d.data_ptr(), self.myo.data_ptr(), ni, nj, nj,
+                     self.pitch)], stream)
+        self.u, pots = pots[:2], pots[2:]
+        ns = len(m._state_names)
+        self.state, self.state_b = pots[:ns], pots[ns:]
         # device address of a tracker's flags -> (flags, padded copy)
         self.act = {}
 
@@ -112,6 +111,10 @@ class _Mirror:
             out.append(self._rows(pad, f, P, nj))
         return out
 
+    @staticmethod
+    def run_copies(copies, stream):
+        _copy_rows(copies, stream)
+
     def swap(self):
         self.u.reverse()
         self.state, self.state_b = self.state_b, self.state
@@ -123,8 +126,8 @@ class _Mirror:
             a.state[i] = t.data_ptr()
             a.state_b[i] = tb.data_ptr()
         a.myo = self.myo.data_ptr()
-        a.weights = self.w.data_ptr()
         a.weights_packed = self.wpack.data_ptr()
+        a.weight_centre = self.centre.data_ptr()
         for k in range(a.n_lat):
             pad = self.act.get(a.lat[k].activated)
             if pad is None:

@@ -1088,7 +1088,8 @@ bool tma_tissue_ok(const fw_step_args *a)
 {
     const int64_t pitch = a->pitch ? a->pitch : a->nj;
     if (pitch < a->nj || pitch % 16 || pitch >= (1 << 30)) return false;
-    if (!aligned16(a->weights_packed) || !aligned16(a->weights) ||
+    if (!aligned16(a->weights_packed) ||
+        !aligned16(a->weight_centre ? (const void *)a->weight_centre : a->weights) ||
         !aligned16(a->u[0]) || !aligned16(a->u[1]) || !aligned16(a->myo))
         return false;
     int ns = 0, np = 0;
@@ -1120,7 +1121,9 @@ int fill_tma_tissue(const fw_step_args *a, int64_t n_begin, BTissueT &T, bool pa
               encode_2d(&T.maps.u[1], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a->u[1],
                         a->nj, a->ni, kBoxF, LH + 2, pitch) &&
               encode_2d(&T.maps.wc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
-                        (const float *)a->weights + (int64_t)cen * a->ni * pitch,
+                        a->weight_centre ? a->weight_centre
+                                         : (const float *)a->weights +
+                                               (int64_t)cen * a->ni * pitch,
                         a->nj, a->ni, kBoxF, LH, pitch);
     // maps of two state arrays in both buffers exist for every tissue (the
     // kernel acquires them); models with one state variable map the first

@@ -91,8 +91,11 @@ int check_step_args(const fw_step_args *a, int64_t n_steps)
         set_error("fw_step: n_steps %lld out of range", (long long)n_steps);
         return FW_ERR_ARG;
     }
-    if (a->pitch != 0 && a->pitch != a->nj) {
-        set_error("fw_step: a row pitch other than nj is for batches only");
+    if (a->pitch != 0 && a->pitch != a->nj &&
+        (a->form != FW_FORM_FUSED || dim != 2 || a->pitch < a->nj ||
+         a->pitch % 16 != 0 || a->pitch >= (1 << 30))) {
+        set_error("fw_step: a row pitch other than nj is for batches and the "
+                  "fused TMA kernels (a multiple of 16, at least nj)");
         return FW_ERR_UNSUPPORTED;
     }
     if (!a->mesh || !a->myo || !a->weights || !a->u[0] || !a->u[1] ||
@@ -285,6 +288,12 @@ int fw_ionic(int32_t model, int32_t precision, void *u_new, const void *u,
         }
     return fw::ionic(model, precision, u_new, u, state, idx, n_idx, dt, params,
                      (cudaStream_t)stream);
+}
+
+int fw_pack_rows(int32_t stencil, const float *w, int64_t ni, int64_t nj,
+                 int64_t pitch, float *out, float *centre, void *stream)
+{
+    return fw::pack_rows(stencil, w, ni, nj, pitch, out, centre, (cudaStream_t)stream);
 }
 
 int fw_nonmyo_differ(const int8_t *myo, const void *u0, const void *u1,

@@ -1230,16 +1230,20 @@ inline int sm_count()
 
 inline bool aligned16(const void *p) { return p && ((uintptr_t)p & 15) == 0; }
 
+// Row pitch of the arrays the TMA kernels read (fw_step_args.pitch).
+inline int64_t row_pitch(const fw_step_args *a) { return a->pitch ? a->pitch : a->nj; }
+
 // True when the TMA form can run this configuration: every array it reads
 // through a tensor map (packed weights, the weights' centre plane, both
 // potential buffers, the myocyte flags, the model's `ns` state arrays and
 // the local activation tracker's flags) starts on a 16-byte boundary, and
-// rows are a multiple of 16 nodes.
+// rows are a multiple of 16 nodes apart.
 inline bool tma_usable(const fw_step_args *a, int ns)
 {
-    bool ok = aligned16(a->weights_packed) && aligned16(a->weights) &&
+    bool ok = aligned16(a->weights_packed) &&
+              aligned16(a->weight_centre ? (const void *)a->weight_centre : a->weights) &&
               aligned16(a->u[0]) && aligned16(a->u[1]) && aligned16(a->myo) &&
-              a->nj % 16 == 0 && a->ni < (1 << 30) && a->nj < (1 << 30);
+              row_pitch(a) % 16 == 0 && a->ni < (1 << 30) && a->nj < (1 << 30);
     for (int q = 0; q < ns && ok; ++q)
         ok = aligned16(a->state[q]) && aligned16(a->state_b[q]);
     for (int l = 0; l < a->n_lat && ok; ++l) ok = aligned16(a->lat[l].activated);
@@ -1284,36 +1288,39 @@ int launch_fused_tma(const fw_step_args *a, int64_t n_begin, int64_t n_steps,
                   kMaxFusedLat);
         return FW_ERR_UNSUPPORTED;
     }
+    const int64_t pitch = row_pitch(a);
     TmaK k;  // kernel argument, copied at each launch
     memset(&k, 0, sizeof k);
     k.force_timeout = (a->debug_flags & FW_DEBUG_FORCE_TIMEOUT) ? 1 : 0;
     bool ok = (FLY ? encode_2d(&k.maps.fib, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
                                a->fibers_f32, 2 * a->nj, a->ni, kBoxFib, LH)
                    : PAIRS ? encode_weights_pairs(&k.maps.w, a->weights_packed, NWO,
-                                                  a->nj, a->ni, LH)
+                                                  a->nj, a->ni, LH, pitch)
                            : encode_weights(&k.maps.w, a->weights_packed, NWO, a->nj,
-                                            a->ni, LH)) &&
+                                            a->ni, LH, pitch)) &&
               encode_2d(&k.maps.myo, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a->myo,
-                        a->nj, a->ni, kBoxB, LH) &&
+                        a->nj, a->ni, kBoxB, LH, pitch) &&
               encode_2d(&k.maps.u[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a->u[0],
-                        a->nj, a->ni, kBoxF, LH + 2) &&
+                        a->nj, a->ni, kBoxF, LH + 2, pitch) &&
               encode_2d(&k.maps.u[1], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a->u[1],
-                        a->nj, a->ni, kBoxF, LH + 2);
+                        a->nj, a->ni, kBoxF, LH + 2, pitch);
     for (int q = 0; q < M::NS && ok; ++q)
         ok = encode_2d(&k.maps.s[0][q], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
-                       a->state[q], a->nj, a->ni, kBoxF, LH) &&
+                       a->state[q], a->nj, a->ni, kBoxF, LH, pitch) &&
              encode_2d(&k.maps.s[1][q], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
-                       a->state_b[q], a->nj, a->ni, kBoxF, LH);
-    // the centre plane of the (nw, ni * nj) float32 weights
+                       a->state_b[q], a->nj, a->ni, kBoxF, LH, pitch);
+    // the centre plane of the (nw, ni * pitch) float32 weights
     if (ok && !FLY) {
-        const float *wcen_plane = (const float *)a->weights +
-                                  (int64_t)Stencil2D<ST>::CENTRE * a->ni * a->nj;
+        const float *wcen_plane =
+            a->weight_centre ? a->weight_centre
+                             : (const float *)a->weights +
+                                   (int64_t)Stencil2D<ST>::CENTRE * a->ni * pitch;
         ok = encode_2d(&k.maps.wc, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, wcen_plane,
-                       a->nj, a->ni, kBoxF, LH);
+                       a->nj, a->ni, kBoxF, LH, pitch);
     }
     if (ok && a->n_lat > 0)
         ok = encode_2d(&k.maps.act, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1,
-                       a->lat[0].activated, a->nj, a->ni, kBoxB, LH);
+                       a->lat[0].activated, a->nj, a->ni, kBoxB, LH, pitch);
     if (!ok) {
         set_error("fw_step (fused TMA): tensor map encoding failed");
         return FW_ERR_UNSUPPORTED;
@@ -1327,7 +1334,7 @@ int launch_fused_tma(const fw_step_args *a, int64_t n_begin, int64_t n_steps,
     f.ni = (int32_t)a->ni;
     f.nj = (int32_t)a->nj;
     f.n = a->ni * a->nj;
-    f.pitch = (int32_t)a->nj;
+    f.pitch = (int32_t)pitch;
     f.status = a->status;
     f.fly_dal = (float)a->fly_D_al;
     f.fly_dac = (float)a->fly_D_ac;
@@ -1403,6 +1410,11 @@ int fused_dispatch(const fw_step_args *a, int64_t n_begin, int64_t n_steps,
             return FW_ERR_ARG;
         }
     if (v == 0) v = tma_usable(a, M::NS) ? 3 : 1;
+    if (row_pitch(a) != a->nj && v != 3 && v != 4 && v != 6) {
+        set_error("fw_step (fused): padded rows need a TMA kernel (fused_variant "
+                  "3, 4 or 6)");
+        return FW_ERR_UNSUPPORTED;
+    }
     if (v == 5) {
         if constexpr (ST == FW_STENCIL_ANISO9) {
             if (!tma_fly_usable(a, M::NS)) {

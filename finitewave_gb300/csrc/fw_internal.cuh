@@ -184,6 +184,8 @@ int ecg(int32_t stencil, int32_t precision, const void *u, const void *w,
         cudaStream_t stream);
 int step_fused(const fw_step_args *a, int64_t n_begin, int64_t n_steps,
                cudaStream_t stream);
+int pack_rows(int32_t stencil, const float *w, int64_t ni, int64_t nj, int64_t pitch,
+              float *out, float *centre, cudaStream_t stream);
 int nonmyo_differ(const int8_t *myo, const void *u0, const void *u1,
                   int32_t precision, int64_t n, int32_t *flag, cudaStream_t stream);
 int copy_rows(const fw_rows *copies, int32_t n, cudaStream_t stream);

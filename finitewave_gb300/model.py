@@ -31,6 +31,10 @@ from .tracker import (ActivationTime2DTracker, ECG2DTracker,
 
 _NP = {"float64": np.float64, "float32": np.float32}
 _MAX_SEGMENT = 1 << 20
+# steps of a segment from which rows of no multiple of 16 nodes run on padded
+# copies, where the tuner, which counts the copies in and out against 96
+# steps, found that faster
+_PAD_MIN_STEPS = 64
 
 
 def _np_name(npfloat):
@@ -320,6 +324,24 @@ class CardiacModel:
         self._pack_weights()
         self._weight_rows()
         self._node_order()
+        self._pad = None
+
+    def _pad_ok(self):
+        """Row-padded copies of the arrays may be kept for the TMA kernels
+        (about 90 bytes a node more; not for a request whose admission
+        counted its own arrays)."""
+        shape = self._shape()
+        return (getattr(self, "pad_rows", True) and
+                len(shape) == 2 and shape[1] % 16 != 0 and
+                self.stencil.kind in (_ffi.ISO5, _ffi.ANISO9) and
+                self._model_id in self._FUSED_MODELS)
+
+    def _padded(self):
+        """The row-padded copies, made once per set of weights."""
+        from .batch import _Mirror
+        if getattr(self, "_pad", None) is None or not self._pad.valid_for(self):
+            self._pad = _Mirror(self)
+        return self._pad
 
     def _node_order(self):
         """The nodes with the myocytes first (fw_step_args.node_list), for
@@ -636,12 +658,37 @@ class CardiacModel:
         status word is not read back (no host synchronisation)."""
         seg = self._prepare_segment(limit)
         stream = torch.cuda.current_stream().cuda_stream
+        pad = self._segment_padding(seg)
+        if pad is not None:
+            pad.run_copies(pad.copies_in(), stream)
+            variant = seg.args.fused_variant
+            pad.apply(seg.args)
+            seg.args.fused_variant = variant
         _ffi.call("fw_step", ctypes.byref(seg.args), seg.n0, seg.n_seg,
                   stream)
         if sync:
             self._check_status()
         self._finish_segment(seg)
+        if pad is not None:
+            if seg.n_seg % 2 == 1:
+                pad.swap()
+            pad.run_copies(pad.copies_out(), stream)
         return seg.n_seg
+
+    def _segment_padding(self, seg):
+        """The padded copies a fused segment runs on, when the tuner chose a
+        TMA kernel for rows of no multiple of 16 nodes and the segment is
+        long enough; a shorter one gets the best kernel on the model's own
+        arrays."""
+        a = seg.args
+        if (a.form != _ffi.FORM_FUSED or a.weights_packed or self.fused_k or
+                self.fused_variant or a.fused_variant not in (3, 4)):
+            return None
+        if self._pad_ok() and seg.n_seg >= _PAD_MIN_STEPS:
+            return self._padded()
+        from . import autotune
+        a.fused_variant, a.fused_k = autotune.choose_flat(self)
+        return None
 
     def _bare_args(self, tune=True):
         """fw_step_args with the model's arrays, parameters and kernel

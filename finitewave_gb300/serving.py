@@ -193,6 +193,7 @@ class SimulationServer:
     def _prepare(self, r):
         """initialize() on the request's stream (worker thread)."""
         m = r.model
+        m.pad_rows = False   # the admission counted the model's own arrays
         with self._ops.using(r._stream):
             m.initialize()
             if m.state_loader:

@@ -294,8 +294,9 @@ typedef struct fw_step_args {
                             local activation trackers' `activated` flags
                             (their N is ni * pitch); 0 = nj.  Stimulus
                             masks and the other tracker arrays always have
-                            rows of nj nodes.  fw_batch_plan only: fw_step
-                            takes 0 or nj                                 */
+                            rows of nj nodes.  fw_step takes a pitch other
+                            than nj (a multiple of 16) in the fused form
+                            with fused_variant 0, 3, 4 or 6               */
     void *state_b[FW_MAX_FUSED_STATE]; /* FW_FORM_FUSED and batches: second
                             buffers of the state variables (same type and
                             size as state[], equal to them at non-myocytes).
@@ -333,6 +334,10 @@ typedef struct fw_step_args {
                             run one thread per myocyte, so no lane of a
                             warp idles on a non-myocyte; same results       */
     int64_t n_list_myo;
+    const float *weight_centre; /* TMA kernels, optional: the centre plane of
+                            the weights, rows `pitch` apart (16-byte
+                            aligned), read instead of the one in `weights`,
+                            which may then keep rows of nj nodes            */
 } fw_step_args;
 
 /* A planned batch of tissues (fw_batch_plan).  Host-side handle; the
@@ -437,6 +442,12 @@ typedef struct fw_rows {
 /* n such copies, any number per launch up to 64 (the tissues of a batch move
  * in and out of their row-padded copies).  The arrays must not overlap. */
 FW_API int fw_copy_rows(const fw_rows *copies, int32_t n, void *stream);
+
+/* The same for rows `pitch` >= nj nodes apart: packs the (nw, ni, nj)
+ * weights into out (ni, pitch, nwo) and their centre plane into centre
+ * (ni, pitch), zeros in the padding. */
+FW_API int fw_pack_rows(int32_t stencil, const float *w, int64_t ni, int64_t nj,
+             int64_t pitch, float *out, float *centre, void *stream);
 
 /* fw_step_args.node_list of a grid: the n < 2^31 nodes with those of
  * myo != 0 first, each part in ascending order, written to list (n).

@@ -85,3 +85,20 @@ def test_bad_arguments(ffi):
     arr = (ffi.Rows * 1)((t.data_ptr(), t.data_ptr() + 128, 2, 16, 8, 16))
     assert lib.fw_copy_rows(arr, 1, None) == -1
     assert lib.fw_copy_rows(None, 0, None) == 0
+
+
+@pytest.mark.parametrize("kind,nw,centre", [(0, 5, 2), (1, 9, 4)])
+@pytest.mark.parametrize("ni,nj", [(1, 1), (3, 17), (40, 255), (5, 1000), (4200, 33)])
+def test_pack_rows(ffi, kind, nw, centre, ni, nj):
+    kind = (ffi.ISO5, ffi.ANISO9)[kind]
+    w = torch.randn((nw, ni, nj), device="cuda")
+    pitch = -(-nj // 16) * 16
+    out = torch.full((ni, pitch, nw - 1), 9.0, device="cuda")
+    cen = torch.full((ni, pitch), 9.0, device="cuda")
+    ffi.call("fw_pack_rows", kind, w.data_ptr(), ni, nj, pitch, out.data_ptr(),
+             cen.data_ptr(), _stream())
+    want = torch.zeros((ni, pitch, nw - 1), device="cuda")
+    want[:, :nj] = w[[q for q in range(nw) if q != centre]].permute(1, 2, 0)
+    c = torch.zeros((ni, pitch), device="cuda")
+    c[:, :nj] = w[centre]
+    assert torch.equal(out, want) and torch.equal(cen, c)
