@@ -7,8 +7,10 @@
 // descriptor table plus a list of (tissue, tile) pairs covering every tissue
 // with the fused form's temporally blocked regions; fw_batch_run then
 // advances all tissues by K time steps per launch.  The CTAs of a launch are
-// persistent (a few per SM) and take tiles from a shared counter in a small
-// caller-provided scratch buffer, so tissues of different models and sizes
+// persistent and take tiles from counters in a small caller-provided scratch
+// buffer -- one per (model, stencil) group, whose CTAs are a share of the
+// launch by the group's work (group_shares) or, in batches of many tiles, a
+// kernel of their own -- so tissues of different models and sizes
 // balance across the GPU; the last CTA to finish resets the counters, so the
 // scratch stays zero between launches.
 //
@@ -566,7 +568,7 @@ constexpr int kGroupKey[kGroups] = {
 
 // Time of a group's tile, in any unit (us measured with one group alone):
 // the groups' parts of the SMs follow it.
-constexpr double kGroupCost[kGroups] = {4.8, 5.0, 5.8, 6.3, 6.8, 7.1};
+constexpr double kGroupCost[kGroups] = {4.7, 5.1, 4.8, 5.3, 6.5, 6.9};
 
 // The per-launch fields of tissue T's launch description: step window masks
 // of the stimuli and trackers, first step, step count and the potential

@@ -289,8 +289,10 @@ __global__ void __launch_bounds__(step_threads<T>(), (MinBlocks<M, T>::value))
     // come only when a CTA is done: placed earlier, in the slots that this
     // step's CTAs leave, they would not spread evenly over the SMs, whose
     // float64 pipes set the time (TP06 192 x 190: 68 against 61 us a step).
-    // One step of Courtemanche float32 511 x 387 takes 6.6 us so, 8.4 without;
-    // of Aliev-Panfilov float32 256 x 240 x 60 59 against 62.
+    // With and without the overlap, us a step: Courtemanche float32 511 x 387
+    // 12.8 and 14.5, Aliev-Panfilov float32 256 x 240 x 60 59.8 and 61.8 and
+    // 320 x 300 4.0 and 5.8 (ECG samples included), float64 600 x 601 with
+    // 20 % fibrosis 28.5 and 30.9.
     constexpr bool kLate = LIST && sizeof(T) == 8;
     if constexpr (!kLate) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
