@@ -131,12 +131,15 @@ def tune(model, steps=96):
             continue
     # rows that are no multiple of 16 nodes: the TMA kernels on row-padded
     # copies of the arrays, the copies in and out counted once in `steps`
-    # steps (777 x 1011 nodes: 25 us; Aliev-Panfilov 2500 x 2501 takes 28.8 us
-    # a step so, 37.5 on its own arrays, 500 x 501 2.8 against 2.1)
+    # steps (777 x 1011 nodes: 39 us, 2500 x 2501 93 us; Aliev-Panfilov
+    # 2500 x 2501 takes 28.0 us a step so, 36.3 on its own arrays, 500 x 501
+    # 2.7 against 2.0)
     flat = min(times, key=times.get)
     cost = dict(times)
+    mir = None
     if model._shape()[1] % 16 and model._pad_ok():
         mir = model._padded()
+    if mir is not None:
         copies = _time_copies(mir, stream)
         mir.apply(a)
         for v, k in _TMA:

@@ -39,7 +39,8 @@ class _Mirror:
         ni, nj = m._shape()
         self.model, self.nj = m, nj
         self.pitch = -(-nj // 16) * 16
-        self.weights_src = m.weights
+        self.weights_src, self.myo_src = m.weights, m._myo_d
+        self.versions = m.weights._version, m._myo_d._version
         dev = m._device()
         f32 = torch.float32
         nwo = 4 if m.stencil.kind == _ffi.ISO5 else 8
@@ -62,7 +63,11 @@ class _Mirror:
         self.act = {}
 
     def valid_for(self, m):
-        return m is self.model and m.weights is self.weights_src
+        """The model's weights and flags are still the tensors that were
+        copied, and nothing has been written into them since."""
+        return (m is self.model and m.weights is self.weights_src and
+                m._myo_d is self.myo_src and
+                (m.weights._version, m._myo_d._version) == self.versions)
 
     def _lat_flags(self):
         seq = self.model.tracker_sequence

@@ -328,7 +328,7 @@ class CardiacModel:
 
     def _pad_ok(self):
         """Row-padded copies of the arrays may be kept for the TMA kernels
-        (about 90 bytes a node more; not for a request whose admission
+        (about 50 bytes a node more; not for a request whose admission
         counted its own arrays)."""
         shape = self._shape()
         return (getattr(self, "pad_rows", True) and
@@ -337,10 +337,15 @@ class CardiacModel:
                 self._model_id in self._FUSED_MODELS)
 
     def _padded(self):
-        """The row-padded copies, made once per set of weights."""
+        """The row-padded copies, made once per set of weights (None where
+        the device has no room for them)."""
         from .batch import _Mirror
         if getattr(self, "_pad", None) is None or not self._pad.valid_for(self):
-            self._pad = _Mirror(self)
+            self._pad = None
+            try:
+                self._pad = _Mirror(self)
+            except torch.cuda.OutOfMemoryError:
+                pass
         return self._pad
 
     def _node_order(self):
@@ -678,14 +683,16 @@ class CardiacModel:
     def _segment_padding(self, seg):
         """The padded copies a fused segment runs on, when the tuner chose a
         TMA kernel for rows of no multiple of 16 nodes and the segment is
-        long enough; a shorter one gets the best kernel on the model's own
-        arrays."""
+        long enough and the device has room for them; else the segment gets
+        the best kernel on the model's own arrays."""
         a = seg.args
         if (a.form != _ffi.FORM_FUSED or a.weights_packed or self.fused_k or
                 self.fused_variant or a.fused_variant not in (3, 4)):
             return None
         if self._pad_ok() and seg.n_seg >= _PAD_MIN_STEPS:
-            return self._padded()
+            pad = self._padded()
+            if pad is not None:
+                return pad
         from . import autotune
         a.fused_variant, a.fused_k = autotune.choose_flat(self)
         return None

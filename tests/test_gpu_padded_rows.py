@@ -100,3 +100,31 @@ def test_pitch_arguments(env):
         a.form, a.fused_variant, a.fused_k, a.pitch = form, variant, 4, pitch
         assert lib.fw_step(ctypes.byref(a), 0, 8, None) != 0
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("change", ["weights", "no room"])
+def test_padded_rows_follow_the_model(env, monkeypatch, change):
+    """Weights written in place between two runs are the next run's weights,
+    and a device without room for the copies runs on the model's arrays."""
+    fg, autotune = env
+    from finitewave_gb300 import batch
+    out = []
+    for pad in (True, False):
+        m = _model(fg, "AlievPanfilov2D", (45, 150), True)
+        m.pad_rows = pad
+        m.initialize()
+        autotune._memo[autotune.key(m)] = {"variant": 3, "k": 4, "flat": [1, 4]}
+        if pad and change == "no room":
+            def no_room(model):
+                raise torch.cuda.OutOfMemoryError("no room")
+            monkeypatch.setattr(batch, "_Mirror", no_room)
+        m.t_max = 0.9
+        m.run(initialize=False)
+        if change == "weights":
+            m.weights.mul_(0.99)
+        m.t_max = 1.8
+        m.run(initialize=False)
+        assert (m._pad is not None) == (pad and change == "weights")
+        out.append([m._dev[k].cpu().numpy().copy() for k in ("u", m._state_names[0])])
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
