@@ -149,8 +149,6 @@ __device__ __forceinline__ double conc_probe(const CPair &c)
 struct ModelTP06 {
     static constexpr int NS = 19, NP = 49;
     static constexpr int kMinBlocksF32 = 4;  // 64 registers, no spills
-    // 700 instructions against 210 bytes a node: bound by memory in float32
-    static constexpr bool kStreamsF32 = true;
     enum {
         ko, cao, nao, Vc, Vsr, Vss, Bufc, Kbufc, Bufsr, Kbufsr, Bufss, Kbufss,
         Vmaxup, Kup, Vrel, k1_, k2_, k3, k4, EC, maxsr, minsr, Vleak, Vxfer, R,

@@ -17,8 +17,6 @@
 //   the caller's buffers then swap roles.
 #pragma once
 
-#include <type_traits>
-
 #include "fw_internal.cuh"
 #include "fw_models.cuh"
 
@@ -108,7 +106,6 @@ struct StepK {
     // n_run threads' worth of them are visited, the first n_myo step
     const int32_t *list;
     int32_t n_run, n_myo;
-    int32_t ahead;   // nodes between a thread's node and what it prefetches
     int64_t step;
     int32_t n_at, n_lat;
     AtK<T> at[FW_MAX_AT];
@@ -186,7 +183,6 @@ struct MinBlocks<M, float, decltype(void(M::kMinBlocksF32))> {
 // Below kListMinNodes (four warps an SM) the step's time is the latency of
 // its loads, to which the list adds one: Aliev-Panfilov float64 100 x 100
 // is 4 % slower with it.
-constexpr int64_t kPrefetchBytes = 96 << 20;   // of the 129 MB L2
 constexpr int64_t kListMinNodes = 152 * 4 * 32;
 template <class M, class T, class = void>
 struct UseList {
@@ -212,68 +208,6 @@ template <class M, class T>
 constexpr int step_blocks()
 {
     return UseList<M, T>::value ? 1 << 26 : 152 * 8;
-}
-
-template <class M, class = void>
-struct StreamsF32 : std::false_type {};
-template <class M>
-struct StreamsF32<M, std::void_t<decltype(M::kStreamsF32)>> : std::true_type {};
-
-template <int ST>
-constexpr int stencil_planes()
-{
-    return ST == FW_STENCIL_ISO5 ? 5 : ST == FW_STENCIL_ISO7 ? 7
-           : ST == FW_STENCIL_ANISO9 ? 9 : 19;
-}
-
-// Bytes of state variable i of a node: ion concentrations take 8 in float32.
-template <class M, class = void>
-struct HasConc : std::false_type {};
-template <class M>
-struct HasConc<M, std::void_t<decltype(M::is_conc(0))>> : std::true_type {};
-template <class M, class T>
-constexpr int state_bytes(int i)
-{
-    if constexpr (HasConc<M>::value) return M::is_conc(i) ? 8 : (int)sizeof(T);
-    else return (int)sizeof(T);
-}
-
-// The float32 steps that prefetch when they read more than L2 keeps: those
-// bound by memory.  Aliev-Panfilov 256 x 240 x 60 (343 MB a step) takes 57 us
-// so, 59 without; TP06 256 x 256 x 40 (446 MB) 98 us in grid order with
-// prefetch, 104 without, 101 through the node list with or without.
-template <class M, class T>
-struct Prefetches {
-    static constexpr bool value =
-        sizeof(T) == 4 && (!UseList<M, T>::value || StreamsF32<M>::value);
-};
-
-// What the step reads of node q from HBM, into L2: each array's line, asked
-// for by the first lane of the warp that many nodes earlier (the pointers are
-// launch constants; a lane per array would index them one by one, and was
-// slower than no prefetch).
-template <class M, int ST, class T>
-__device__ __forceinline__ void prefetch_node(const StepK<M, T> &k, int64_t q)
-{
-    if (q + k.si >= k.n) return;
-    auto line = [](const void *p) {
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-    };
-    line(k.u + q + k.si);
-    if (ST == FW_STENCIL_ANISO19_XY && k.wrow) {
-        line(k.widx + q);
-    } else {
-#pragma unroll
-        for (int w = 0; w < stencil_planes<ST>(); ++w)
-            if (ST != FW_STENCIL_ANISO19_XY || w < 9 || w == 11 || w == 12)
-                line(k.w + w * k.n + q);
-    }
-#pragma unroll
-    for (int i = 0; i < M::NS; ++i) {
-        const int b = state_bytes<M, T>(i);
-        line((const char *)k.state[i] + q * b);
-        if (b > (int)sizeof(T) && q + 32 < k.n) line((const char *)k.state[i] + q * b + 128);
-    }
 }
 
 template <class M, int ST, class T, bool LIST>
@@ -308,9 +242,6 @@ __global__ void __launch_bounds__(step_threads<T>(), (MinBlocks<M, T>::value))
         const int64_t p = LIST ? (int64_t)k.list[t] : t;
         T uc = k.u[p];
         if (k.n_at | k.n_lat) track(k, p, uc);
-        if constexpr (Prefetches<M, T>::value)
-            if (k.ahead && (threadIdx.x & 31) == 0)
-                prefetch_node<M, ST, T>(k, p + k.ahead);
         if (LIST ? t >= k.n_myo : !k.myo[p]) continue;
         T un;
         if constexpr (ST == FW_STENCIL_ANISO19_XY) {
@@ -704,19 +635,11 @@ int run_plain(const fw_step_args *a, int64_t n_begin, int64_t n_steps,
     }
 
     constexpr int threads = step_threads<T>();
-    // a float32 step that reads more than L2 keeps for the next prefetches as
-    // many nodes ahead as are under way at a time; TP06 (M::kStreamsF32), then
-    // bound by memory, visits the grid in order, in whole lines
-    const bool large = sizeof(T) == 4 &&
-                       g.n * (int64_t)sizeof(T) * (1 + M::NS + stencil_planes<ST>()) >
-                           kPrefetchBytes;
     const bool listed = UseList<M, T>::value && a->node_list &&
-                        g.n >= kListMinNodes && !(large && StreamsF32<M>::value);
-    k.ahead = large ? 152 * 8 * threads : 0;   // the loop's next node
+                        g.n >= kListMinNodes;
     k.list = listed ? a->node_list : nullptr;
     k.n_myo = (int32_t)a->n_list_myo;
-    const int blocks_all = grid_for(
-        g.n, threads, listed ? step_blocks<M, T>() : 152 * 8 * (kThreads / threads));
+    const int blocks_all = grid_for(g.n, threads, step_blocks<M, T>());
     const int blocks_myo = grid_for(a->n_list_myo, threads, step_blocks<M, T>());
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -76,38 +76,3 @@ def test_listed_steps_equal_grid_order(fg, cls, npfloat, shape, special):
                    [t.output for t in trs])
     for a, b in zip(*out):
         assert np.array_equal(a, b)
-
-
-@pytest.mark.parametrize("cls,shape", [("AlievPanfilov3D", (150, 131, 70)),
-                                       ("TP063D", (120, 110, 66)),
-                                       ("FentonKarma2D", (1900, 1777))])
-def test_steps_larger_than_l2(fg, cls, shape):
-    """float32 steps above the prefetch size (and one below it, 2D) against
-    the same steps on a half of the grid that stays below it: nodes further
-    than the steps from the cut agree bit for bit."""
-    gen = np.random.default_rng(4)
-    mesh = np.where(gen.random(shape) < 0.1, 2, 1).astype(np.int8)
-    half = shape[0] // 2
-    detailed = cls.startswith("TP06")
-    u = gen.random(shape) * (100.0 if detailed else 1.0) - (85.0 if detailed else 0.0)
-    out = []
-    for sl in (slice(None), slice(0, half)):
-        part = mesh[sl]
-        tissue = (fg.CardiacTissue2D if len(shape) == 2 else fg.CardiacTissue3D)(part.shape)
-        tissue.mesh = part.copy()
-        m = getattr(fg, cls)()
-        m.dt, m.dr, m.t_max, m.npfloat = 0.01, 0.25, 0.055, "float32"
-        m.form = "plain"
-        if len(shape) == 3:
-            ang = np.random.default_rng(6).uniform(-1, 1, part.shape[2])
-            f = np.zeros(part.shape + (3,))
-            f[..., 0], f[..., 1] = np.cos(ang), np.sin(ang)
-            tissue.fibers = f
-        m.cardiac_tissue = tissue
-        m.initialize()
-        m.u = u[sl]
-        m.run(initialize=False)
-        out.append([getattr(m, n) for n in ["u"] + list(m._state_names)])
-    keep = slice(0, half - 8)   # 6 steps, one node a step, and the cut's ring
-    for a, b in zip(*out):
-        assert np.array_equal(a[keep], b[keep])
