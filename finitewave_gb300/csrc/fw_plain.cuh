@@ -178,8 +178,9 @@ struct MinBlocks<M, float, decltype(void(M::kMinBlocksF32))> {
 // whatever the number of myocytes among its nodes.  Measured with 10-20 %
 // fibrosis, list and one-warp CTAs against grid order and 256 threads:
 // Aliev-Panfilov float64 600 x 601 30 against 35 us a step, TP06 float64
-// 192 x 190 150 against 169, Courtemanche float32 511 x 387 10.4 against
-// 12.0, TP06 float32 256 x 256 x 40 107 against 112.
+// 192 x 190 150 against 169 (reference-order update); with 256 threads on
+// both sides, Courtemanche float32 511 x 387 12.8 against 13.6, TP06 float32
+// 192^3 shell (19 % myocytes) 83 against 105.
 // Below kListMinNodes (four warps an SM) the step's time is the latency of
 // its loads, to which the list adds one: Aliev-Panfilov float64 100 x 100
 // is 4 % slower with it.
@@ -195,7 +196,15 @@ struct UseList<M, T, decltype(void(M::kMinBlocksF32))> {
 
 // Threads per CTA.  float64 steps are bound by the float64 pipe, so what
 // counts is that every SM gets the same number of warps: one-warp CTAs, as
-// many as the grid has, go to whichever SM is free.
+// many as the grid has, go to whichever SM is free.  Listed float32 steps
+// launch kListThreadsF32 of the kThreads that the kernel is compiled for (its
+// registers and the threads an SM holds stay as they are): the same fill, in
+// halves, leaves less of the last round empty.  Us a step with 256, 128 and
+// 64: Courtemanche 511 x 387 12.8, 12.0, 12.1, 700 x 700 24.2, 22.4, 22.4;
+// TP06 500 x 501 10.6, 9.9, 9.9, 256 x 256 x 40 106, 104, 103, 100 x 100 x 20
+// 9.5, 8.5, 8.7, 192^3 shell 83.0, 83.2, 83.9; with 32 TP06 500 x 501 takes
+// 11.8 (an SM holds 32 CTAs at most).
+constexpr int kListThreadsF32 = 128;
 template <class T>
 constexpr int step_threads()
 {
@@ -634,9 +643,9 @@ int run_plain(const fw_step_args *a, int64_t n_begin, int64_t n_steps,
         if (fw_state_is_pair(a->model, a->precision, i)) pk.pair_mask |= 1u << i;
     }
 
-    constexpr int threads = step_threads<T>();
     const bool listed = UseList<M, T>::value && a->node_list &&
                         g.n >= kListMinNodes;
+    const int threads = sizeof(T) == 4 && listed ? kListThreadsF32 : step_threads<T>();
     k.list = listed ? a->node_list : nullptr;
     k.n_myo = (int32_t)a->n_list_myo;
     const int blocks_all = grid_for(g.n, threads, step_blocks<M, T>());
