@@ -135,7 +135,7 @@ int pack_rows(int32_t stencil, const float *w, int64_t ni, int64_t nj, int64_t p
 namespace {
 
 // 16 nodes a thread and round: their flags in one load, and the potentials
-// only of groups that hold a non-myocyte.  Bound by memory: 26 us on 4096^2
+// only of groups that hold a non-myocyte.  Bound by memory: 42 us on 4096^2
 // nodes at 20 % fibrosis, where index, gather and compare of whole arrays
 // took 250 us and four host synchronisations.
 template <class T>

@@ -19,8 +19,9 @@
 // weights' own centre plane beside the packed off-centre weights (9 FMA per
 // node and sub-step instead of 17 operations for  u + sum_k w_k (u_k - u)).
 //
-// Layout requirements (checked by the host): nj % 16 == 0 (TMA row strides
-// and the int8 myocyte rows) and the packed weight array of fw_pack_weights.
+// Layout requirements (checked by the host): rows a multiple of 16 nodes
+// apart, nj itself or the caller's padded pitch (TMA row strides and the int8
+// myocyte rows), and the packed weight array of fw_pack_weights.
 // Boxes start at 16-byte aligned x coordinates (x rounded down, the data is
 // addressed at an offset inside the box), negative and past-the-end
 // coordinates read zeros.

@@ -443,12 +443,6 @@ typedef struct fw_rows {
  * in and out of their row-padded copies).  The arrays must not overlap. */
 FW_API int fw_copy_rows(const fw_rows *copies, int32_t n, void *stream);
 
-/* The same for rows `pitch` >= nj nodes apart: packs the (nw, ni, nj)
- * weights into out (ni, pitch, nwo) and their centre plane into centre
- * (ni, pitch), zeros in the padding. */
-FW_API int fw_pack_rows(int32_t stencil, const float *w, int64_t ni, int64_t nj,
-             int64_t pitch, float *out, float *centre, void *stream);
-
 /* fw_step_args.node_list of a grid: the n < 2^31 nodes with those of
  * myo != 0 first, each part in ascending order, written to list (n).
  * scratch: device int32, n / 4096 + 2 values. */
@@ -461,6 +455,12 @@ FW_API int fw_node_list(const int8_t *myo, int64_t n, int32_t *list,
  * implied because each stencil row sums to one).  2D stencils only. */
 FW_API int fw_pack_weights(int32_t stencil, const float *w, int64_t n,
                            float *out, void *stream);
+
+/* The same for rows `pitch` >= nj nodes apart: packs the (nw, ni, nj)
+ * weights into out (ni, pitch, nwo) and their centre plane into centre
+ * (ni, pitch), zeros in the padding. */
+FW_API int fw_pack_rows(int32_t stencil, const float *w, int64_t ni, int64_t nj,
+             int64_t pitch, float *out, float *centre, void *stream);
 
 /* One ECG sample: the sum of fw_ecg_tracker for the potential u (N nodes)
  * with weights w (nw, N) over the nodes with myo[p] != 0, for n_leads
