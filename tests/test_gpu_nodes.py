@@ -76,3 +76,41 @@ def test_listed_steps_equal_grid_order(fg, cls, npfloat, shape, special):
                    [t.output for t in trs])
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("cls,npfloat,shape", [
+    ("AlievPanfilov2D", "float64", (141, 150)), ("TP062D", "float32", (141, 150))])
+@pytest.mark.parametrize("start,step", [(0, 1), (0.04, 1), (0.03, 2), (0, 3)])
+def test_listed_activation_at_non_myocytes(fg, cls, npfloat, shape, start, step):
+    """Non-myocytes above the threshold in either potential buffer, trackers
+    whose windows open late or skip steps: the activation steps are those of
+    grid order."""
+    out = []
+    for listed in (True, False):
+        gen = np.random.default_rng(5)
+        t = fg.CardiacTissue2D(shape)
+        t.mesh = np.where(gen.random(shape) < 0.3, 2, 1).astype(np.int8)
+        m = getattr(fg, cls)()
+        m.dt, m.dr, m.npfloat, m.cardiac_tissue = 0.01, 0.25, npfloat, t
+        seq = fg.StimSequence()
+        seq.add_stim(fg.StimVoltageCoord2D(0.05, 1.0, 20, 90, 20, 90))
+        m.stim_sequence = seq
+        trs = fg.TrackerSequence()
+        for thr in (0.5, 0.8):
+            tr = fg.ActivationTime2DTracker()
+            tr.threshold = thr
+            trs.add_tracker(tr)
+        trs.sequence[1].start_time, trs.sequence[1].step = start, step
+        m.tracker_sequence = trs
+        m.t_max = 0.115
+        m.initialize()
+        for name in ("u", "u_new"):
+            u = m._dev[name]
+            r = torch.as_tensor(gen.random(shape), device=u.device, dtype=u.dtype)
+            u.copy_(torch.where(m._myo_d.reshape(shape) == 0, r, u))
+        if not listed:
+            m._nodes = None
+        m.run(initialize=False)
+        out.append([np.asarray(tr.output) for tr in trs.sequence])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b) and (a >= 0).any()
