@@ -220,11 +220,12 @@ __device__ __forceinline__ double ex(double x)
     return ex_scaled(x, 1.0, (float)(256 * kLog2e));
 }
 
-// x limited to [-690, 690] (finite x), on the bits
+// x limited to [-690, 690], on the bits; a NaN (quiet, as arithmetic makes
+// them: its high word is above infinity's) stays one
 __device__ __forceinline__ double limited(double x)
 {
-    const int hi = __double2hiint(x);
-    if ((hi & 0x7fffffff) > 0x40859000)
+    const int hi = __double2hiint(x), a = hi & 0x7fffffff;
+    if (a > 0x40859000 && a <= 0x7ff00000)
         x = __hiloint2double((hi & 0x80000000) | 0x40859000, 0);
     return x;
 }
@@ -387,11 +388,17 @@ __device__ __forceinline__ float gate_to(float x, float inf, float decay)
 }
 
 // x / (e^x - 1), given e = e^x.  float64: as it stands, like the models'
-// expressions.  float32: the series of the Bernoulli numbers up to |x| = 1/2
-// (next term x^10 / 47900160), where the difference would lose digits.
+// expressions, and like theirs NaN at x = 0 and infinite where e rounds to 1
+// (Courtemanche's beta_xr at the potential next above 3.3328 mV).  float32:
+// the series of the Bernoulli numbers up to |x| = 1/2 (next term
+// x^10 / 47900160), where the difference would lose digits.
 __device__ __forceinline__ double x_over_expm1(double x, double e)
 {
-    return x * rcp(e - 1.0);
+    const double d = e - 1.0;
+    double y = rcp(d);   // NaN for d = 0
+    if ((__double2hiint(d) | __double2loint(d)) == 0)
+        y = __hiloint2double(0x7ff00000, 0);
+    return x * y;
 }
 __device__ __forceinline__ float x_over_expm1(float x, float e)
 {

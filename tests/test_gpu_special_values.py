@@ -1,0 +1,103 @@
+"""GPU: the models' updates at potentials, parameters and time steps where an
+expression of theirs has no finite value, against the CPU oracle's."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def fg():
+    if not torch.cuda.is_available():
+        pytest.fail("CUDA device required for -m gpu tests")
+    import finitewave_gb300 as fg
+    return fg
+
+
+def _node_update(fg, model, prec, u, state, dt=0.01, **params):
+    """One fw_ionic pass over the nodes; returns the host values of u and the
+    state."""
+    m = getattr(fg, model)()
+    m.npfloat = prec
+    for k, v in params.items():
+        setattr(m, k, v)
+    t = np.float64 if prec == "float64" else np.float32
+    uu = torch.as_tensor(u.astype(t), device="cuda")
+    un = uu.clone()
+    arrs = []
+    for i, name in enumerate(m._state_names):
+        if fg._ffi.state_is_pair(m._model_id, m._precision(), i):
+            from finitewave_gb300.model import _split_pair
+            arrs.append(torch.as_tensor(_split_pair(state[name]), device="cuda"))
+        else:
+            arrs.append(torch.as_tensor(state[name].astype(t), device="cuda"))
+    ptr = (ctypes.c_void_p * len(arrs))(*[a.data_ptr() for a in arrs])
+    par = (ctypes.c_double * len(m._param_names))(*m._params())
+    idx = torch.arange(u.size, device="cuda")
+    fg._ffi.call("fw_ionic", m._model_id, m._precision(), un.data_ptr(),
+                 uu.data_ptr(), ptr, idx.data_ptr(), u.size, dt, par,
+                 torch.cuda.current_stream().cuda_stream)
+    out = {"u": un.cpu().numpy().astype(np.float64)}
+    for name, a in zip(m._state_names, arrs):
+        a = a.cpu().numpy().astype(np.float64)
+        out[name] = a[:, 0] + a[:, 1] if a.ndim == 2 else a
+    return out
+
+
+def _oracle_update(oracle, name, u, state, **params):
+    un = u.copy()
+    st = {k: v.copy() for k, v in state.items()}
+    with np.errstate(all="ignore"):
+        oracle._ionic(name, st, un, u, np.arange(u.size), 0.01,
+                      dict(oracle.MODELS[name]["params"], **params))
+    return dict(st, u=un)
+
+
+def _state(fg, model, n):
+    """Gates of 0.1 and the initial concentrations."""
+    m = getattr(fg, model)()
+    return {s: np.full(n, float(getattr(m, "init_" + m._init_names.get(s, s)))
+                       if fg._ffi.state_is_pair(m._model_id, fg._ffi.F32, i) else 0.1)
+            for i, s in enumerate(m._state_names)}
+
+
+# potentials at which a rate or a current is 0 / 0
+# (Courtemanche's alpha_m has its limit written out at -47.13)
+POLES = [("Courtemanche2D", "crn", [-14.1, 3.3328, 19.9, -10.0, 7.9, -47.13], 5),
+         ("LuoRudy912D", "lr91", [-47.13, -77.0], 2), ("TP062D", "tp06", [15.0], 1)]
+
+
+@pytest.mark.parametrize("model,name,poles,nans", POLES)
+def test_float64_poles(fg, oracle, model, name, poles, nans):
+    """At the pole itself every variable is NaN exactly where the
+    reference-order update's is, and right next to it finite exactly where
+    that one's is."""
+    p = np.array(poles)
+    u = np.concatenate([p, np.nextafter(p, -1e3), np.nextafter(p, 1e3), p + 1e-9])
+    state = _state(fg, model, u.size)
+    got = _node_update(fg, model, "float64", u, state)
+    want = _oracle_update(oracle, name, u, state)
+    assert np.any([np.isnan(w) for w in want.values()], axis=0).sum() == nans
+    for k in want:
+        assert np.array_equal(np.isnan(got[k]), np.isnan(want[k])), k
+        assert np.array_equal(np.isfinite(got[k]), np.isfinite(want[k])), k
+    # away from the pole by 1e-9 a difference quotient keeps six digits
+    for k in want:
+        a, b = got[k][-p.size:], want[k][-p.size:]
+        assert np.all(np.abs(a - b) <= 1e-5 * np.maximum(1, np.abs(b))), k
+
+
+def test_pole_warns(fg):
+    """A stimulus that sets such a potential is reported by the run."""
+    t = fg.CardiacTissue2D((12, 13))
+    m = fg.Courtemanche2D()
+    m.dt, m.dr, m.t_max, m.cardiac_tissue = 0.01, 0.25, 0.01, t
+    seq = fg.StimSequence()
+    seq.add_stim(fg.StimVoltageCoord2D(0, -10.0, 0, 12, 0, 13))
+    m.stim_sequence = seq
+    with pytest.warns(RuntimeWarning, match="inf or NaN"):
+        m.run()
+    assert np.isnan(np.asarray(m.u)[1:-1, 1:-1]).all()
