@@ -24,10 +24,30 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <initializer_list>
+
 #include "fw_math.cuh"
 #include "fw_models.cuh"
 
 namespace fw {
+
+// Host: the |u| below which an in-range update holds for a model's n
+// parameters: 300 mV, less where an exponent slope * (|u| + u0) that they
+// scale would leave 40, and 0 -- the reference-order update everywhere --
+// where one of them is infinite, NaN or above 1e30, or one of `divisors`, by
+// which a quotient is taken (dm::rcp needs a finite divisor other than zero,
+// and a user may block a pump with a half-saturation of infinity), is not
+// within 1e-30 .. 1e30.
+inline double range_limit(const double *p, int n, std::initializer_list<int> divisors,
+                          double slope, double u0)
+{
+    for (int i = 0; i < n; ++i)
+        if (!(fabs(p[i]) <= 1e30)) return 0.0;
+    for (int i : divisors)
+        if (!(p[i] >= 1e-30)) return 0.0;
+    const double lim = 40.0 / slope - u0;
+    return lim < 300.0 ? lim : 300.0;
+}
 
 // Transcendentals of the reference-order updates.  float64: CUDA's exp / log / pow
 // (the reference's expressions, within a few ulp of the C library).
@@ -244,7 +264,7 @@ struct ModelTP06 {
     // per node and step otherwise).
     enum {
         d_pkn = NP, d_gkr, d_kz, d_cal, d_kw, d_ncx, d_nao3, d_nak, d_naf,
-        d_ssf, d_vcss, d_vsrss, d_ec2, d_kup2, d_dsr, d_end
+        d_ssf, d_vcss, d_vsrss, d_ec2, d_kup2, d_dsr, d_lim, d_end
     };
     static constexpr int ND = d_end - NP;
     static void derive(const double *p, double dt, double *q)
@@ -268,6 +288,13 @@ struct ModelTP06 {
         q[d_ec2] = p[EC] * p[EC];
         q[d_kup2] = p[Kup] * p[Kup];
         q[d_dsr] = p[maxsr] - p[minsr];
+        // exponents z = (u - 15) d_kz, n u d_kw, (n - 1) u d_kw and u d_kw,
+        // d_kw = d_kz / 2
+        const double n = fmax(fmax(fabs(p[n_]), fabs(p[n_] - 1.0)), 2.0);
+        q[d_lim] = range_limit(p, NP,
+                               {Vc, Vss, Kbufsr, Kbufss, Kup, k3, EC, maxsr, minsr, R, F,
+                                T_, KmK, KmNa, KmNai, KmCa, KpCa, ko, cao, nao},
+                               q[d_kw] * n, 15.0);
     }
 
     // ionic_kernel_2d and the calc_* helpers (tp06_2d.py:242-1103)
@@ -277,17 +304,18 @@ struct ModelTP06 {
     {
         const T Ek = P.v[RTONF] * dm::lg(dm::quotient(P.v[ko], (T)x.Ki));
         // the range in which no exponential or product of them below leaves
-        // T's (the squares (u + 25)^2 / 170 and the like set |u| < 300)
-        if (in_range(u, u - Ek)) return update_in_range<T>(u, un, x, P, dt, Ek);
+        // T's (the squares (u + 25)^2 / 170 and the like set |u| < 300, which
+        // is d_lim for parameters as they come)
+        if (in_range(u, u - Ek, P.v[d_lim])) return update_in_range<T>(u, un, x, P, dt, Ek);
         return update_any<T>(u, un, x, P, dt);
     }
-    __device__ static __forceinline__ bool in_range(double u, double x)
+    __device__ static __forceinline__ bool in_range(double u, double x, double lim)
     {
-        return fabs(u) < 300.0 && x > -400.0 && x < 1000.0;
+        return fabs(u) < lim && x > -400.0 && x < 1000.0;
     }
-    __device__ static __forceinline__ bool in_range(float u, float x)
+    __device__ static __forceinline__ bool in_range(float u, float x, float lim)
     {
-        return fabsf(u) < 130.f && x > -100.f && x < 1000.f;
+        return fabsf(u) < fminf(lim, 130.f) && x > -100.f && x < 1000.f;
     }
 
     // The update with few divisions and exponentials, in either precision:
@@ -816,7 +844,7 @@ struct ModelCRN {
 
     enum {
         d_rtf = NP, d_rtf2, d_kw, d_nak, d_ncx, d_nao3, d_leak, d_rfv, d_vru, d_upj,
-        d_relj, d_fnr, d_fni, d_t1, d_t2, d_cs, d_end
+        d_relj, d_fnr, d_fni, d_t1, d_t2, d_cs, d_lim, d_end
     };
     static constexpr int ND = d_end - NP;
     static void derive(const double *p, double, double *q)
@@ -841,6 +869,12 @@ struct ModelCRN {
         q[d_t1] = p[trpnmax] * p[kmtrpn];
         q[d_t2] = p[cmdnmax] * p[kmcmdn];
         q[d_cs] = p[csqnmax] * p[kmcsqn];
+        // exponents up to u d_kw, and nao / 67.3
+        q[d_lim] = range_limit(p, NP,
+                               {F, T_, R, Vj, Vup, caupmax, kup, kmnai, kmko, kmnancx,
+                                kmcancx, kmcmdn, kmtrpn, kmcsqn, cao, nao, ko},
+                               q[d_kw], 0.0);
+        if (p[nao] > 40.0 * 67.3) q[d_lim] = 0.0;
     }
 
     // ionic_kernel_2d and its helpers (courtemanche_2d.py:180-641)
@@ -855,11 +889,10 @@ struct ModelCRN {
             // differs by 1e-3 there
             return update_ref<T>(u, un, x, P, dt);
         } else {
-            if (in_range(u)) return update_in_range<T>(u, un, x, P, dt);
+            if (fabs(u) < P.v[d_lim]) return update_in_range<T>(u, un, x, P, dt);
             return update_any<T>(u, un, x, P, dt);
         }
     }
-    __device__ static __forceinline__ bool in_range(double u) { return fabs(u) < 300.0; }
 
     // As ModelTP06::update_in_range (float64 only): one quotient per rate.
     // 192 x 190 nodes: 65 against 180 us a step.

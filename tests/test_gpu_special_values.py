@@ -101,3 +101,39 @@ def test_pole_warns(fg):
     with pytest.warns(RuntimeWarning, match="inf or NaN"):
         m.run()
     assert np.isnan(np.asarray(m.u)[1:-1, 1:-1]).all()
+
+
+# a pump blocked by an infinite half-saturation, constants of zero, and a
+# temperature at which the reversal exponents leave the in-range update's
+PARAMS = [("TP062D", "tp06", dict(Kup=np.inf)), ("TP062D", "tp06", dict(KpCa=np.inf)),
+          ("TP062D", "tp06", dict(k3=0.0, EC=0.0)),
+          ("TP062D", "tp06", dict(gna=0.0, gto=0.0)), ("TP062D", "tp06", dict(T=3.0)),
+          ("TP062D", "tp06", dict(n_=40.0)),
+          ("Courtemanche2D", "crn", dict(kmnai=0.0)), ("Courtemanche2D", "crn", dict(kup=np.inf)),
+          ("Courtemanche2D", "crn", dict(T=3.0)), ("Courtemanche2D", "crn", dict(caupmax=np.inf)),
+          ("Courtemanche2D", "crn", dict(nao=5e4))]
+
+
+# (float32 leaves its own range at T = 3 and n = 40 in any order)
+@pytest.mark.parametrize("model,name,params,prec",
+                         [(*p, "float64") for p in PARAMS] +
+                         [(*p, "float32") for p in PARAMS[:4]])
+def test_unusual_parameters(fg, oracle, model, name, params, prec):
+    """One step with such parameters: finite where the reference-order update
+    is, with the value it has there."""
+    assert all(v in oracle.MODELS[name]["params"] for v in params)
+    u = np.linspace(-95.0, 60.0, 700).astype(np.float32).astype(np.float64)
+    state = _state(fg, model, u.size)
+    if prec == "float32":
+        state = {k: v.astype(np.float32).astype(np.float64) for k, v in state.items()}
+    got = _node_update(fg, model, prec, u, state, **params)
+    want = _oracle_update(oracle, name, u, state, **params)
+    assert any(np.isfinite(w).all() for w in want.values())
+    # float64: exponents up to 4e3 carry half an ulp of themselves; float32:
+    # 1e-3 of a value is far above one step's error, far below a lost term
+    tol = 1e-9 if prec == "float64" else 1e-3
+    for k in want:
+        w, g = want[k], got[k]
+        fine = np.isfinite(w)
+        assert np.array_equal(np.isfinite(g), fine), k
+        assert np.all(np.abs(g - w)[fine] <= tol * np.maximum(1.0, np.abs(w[fine]))), k
