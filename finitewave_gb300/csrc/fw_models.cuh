@@ -437,6 +437,12 @@ struct ModelBO {
         d_fi, d_o1, d_o2, d_so1, d_dso, d_kso, d_si, d_end
     };
     static constexpr int ND = d_end - NP;
+    // (tau2 - tau1) / dt, and 0 where tau1 / dt is beyond float32 (dt = 0):
+    // the quotient is then 0 whatever the sigmoid, not infinity less infinity
+    static double slope(double d_tau, double tau1, double dt)
+    {
+        return fabs(tau1 / dt) < 3e38 ? d_tau / dt : 0.0;
+    }
     static void derive(const double *p, double dt, double *q)
     {
         q[d_v1] = dt / p[tau_v1_m];
@@ -445,7 +451,7 @@ struct ModelBO {
         q[d_wi] = 1.0 / p[tau_w_inf];
         // dt / tau_w_m = 1 / (d_w1 + d_dw sigmoid), and tau_so likewise
         q[d_w1] = p[tau_w1_m] / dt;
-        q[d_dw] = (p[tau_w2_m] - p[tau_w1_m]) / dt;
+        q[d_dw] = slope(p[tau_w2_m] - p[tau_w1_m], p[tau_w1_m], dt);
         q[d_kw] = -2.0 * p[k_w_m] * dm::kLog2e;
         q[d_wp] = dt / p[tau_w_p];
         q[d_s1] = dt / p[tau_s1];
@@ -455,7 +461,7 @@ struct ModelBO {
         q[d_o1] = dt / p[tau_o1];
         q[d_o2] = dt / p[tau_o2];
         q[d_so1] = p[tau_so1] / dt;
-        q[d_dso] = (p[tau_so2] - p[tau_so1]) / dt;
+        q[d_dso] = slope(p[tau_so2] - p[tau_so1], p[tau_so1], dt);
         q[d_kso] = -2.0 * p[k_so] * dm::kLog2e;
         q[d_si] = dt / p[tau_si];
     }

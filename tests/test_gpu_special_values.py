@@ -137,3 +137,23 @@ def test_unusual_parameters(fg, oracle, model, name, params, prec):
         fine = np.isfinite(w)
         assert np.array_equal(np.isfinite(g), fine), k
         assert np.all(np.abs(g - w)[fine] <= tol * np.maximum(1.0, np.abs(w[fine]))), k
+
+
+@pytest.mark.parametrize("prec", ["float64", "float32"])
+@pytest.mark.parametrize("model", ["BuenoOrovio2D", "TP062D", "Courtemanche2D", "LuoRudy912D"])
+def test_step_of_zero(fg, model, prec):
+    """An ionic pass with dt = 0 changes no potential and no gate that is
+    integrated (the others go to the value they have at dt = 0: themselves)."""
+    m = getattr(fg, model)()
+    n = 500
+    u = np.linspace(0.0, 1.5, n) if model == "BuenoOrovio2D" else np.linspace(-95, 60, n)
+    u = u.astype(np.float32).astype(np.float64)
+    state = {k: v.astype(np.float32).astype(np.float64)
+             for k, v in _state(fg, model, n).items()}
+    got = _node_update(fg, model, prec, u, state, dt=0.0)
+    assert np.array_equal(got["u"], u)
+    for k in m._state_names:
+        if k not in ("oo", "irel"):   # algebraic: not integrated
+            # one rounding where a new value is formed as inf - (inf - x)
+            eps = 2.0 ** -50 if prec == "float64" else 2.0 ** -21
+            assert np.all(np.abs(got[k] - state[k]) <= eps * np.maximum(1, np.abs(state[k]))), k
