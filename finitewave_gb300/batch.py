@@ -40,34 +40,46 @@ class _Mirror:
         self.model, self.nj = m, nj
         self.pitch = -(-nj // 16) * 16
         self.weights_src, self.myo_src = m.weights, m._myo_d
-        self.versions = m.weights._version, m._myo_d._version
         dev = m._device()
         f32 = torch.float32
         nwo = 4 if m.stencil.kind == _ffi.ISO5 else 8
         self.wpack = torch.empty(ni * self.pitch * nwo, dtype=f32, device=dev)
         self.centre = torch.empty((ni, self.pitch), dtype=f32, device=dev)
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        _ffi.call("fw_pack_rows", m.stencil.kind, m.weights.data_ptr(), ni, nj,
-                  self.pitch, self.wpack.data_ptr(), self.centre.data_ptr(),
-                  stream)
         # the tensor maps end at column nj - 1: the padding is never read,
         # except the pair view's weights, which are zero there
         self.myo, *pots = (torch.empty((ni, self.pitch), dtype=t, device=dev)
                            for t in [torch.int8] + [f32] * (2 + 2 * len(m._state_names)))
-        _copy_rows([(m._myo_d.data_ptr(), self.myo.data_ptr(), ni, nj, nj,
-                     self.pitch)], stream)
         self.u, pots = pots[:2], pots[2:]
         ns = len(m._state_names)
         self.state, self.state_b = pots[:ns], pots[ns:]
         # device address of a tracker's flags -> (flags, padded copy)
         self.act = {}
+        self.versions = None
+        self.refresh()
 
     def valid_for(self, m):
         """The model's weights and flags are still the tensors that were
-        copied, and nothing has been written into them since."""
+        copied."""
         return (m is self.model and m.weights is self.weights_src and
-                m._myo_d is self.myo_src and
-                (m.weights._version, m._myo_d._version) == self.versions)
+                m._myo_d is self.myo_src)
+
+    def refresh(self):
+        """Copy the weights and flags again where something has been written
+        into them since, or may have been: tensors of inference mode do not
+        count their writes."""
+        m, versions = self.model, None
+        if not (m.weights.is_inference() or m._myo_d.is_inference()):
+            versions = m.weights._version, m._myo_d._version
+            if versions == self.versions:
+                return
+        ni, nj = m._shape()
+        stream = torch.cuda.current_stream(m._device()).cuda_stream
+        _ffi.call("fw_pack_rows", m.stencil.kind, m.weights.data_ptr(), ni, nj,
+                  self.pitch, self.wpack.data_ptr(), self.centre.data_ptr(),
+                  stream)
+        _copy_rows([(m._myo_d.data_ptr(), self.myo.data_ptr(), ni, nj, nj,
+                     self.pitch)], stream)
+        self.versions = versions
 
     def _lat_flags(self):
         seq = self.model.tracker_sequence
@@ -185,6 +197,8 @@ class TissueBatch:
         if mir is None or not mir.valid_for(m):
             mir = _Mirror(m)
             self._mirrors[id(m)] = mir
+        else:
+            mir.refresh()
         return mir
 
     def add(self, model):

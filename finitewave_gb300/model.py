@@ -346,6 +346,8 @@ class CardiacModel:
                 self._pad = _Mirror(self)
             except torch.cuda.OutOfMemoryError:
                 pass
+        else:
+            self._pad.refresh()
         return self._pad
 
     def _node_order(self):

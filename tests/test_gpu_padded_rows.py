@@ -128,3 +128,27 @@ def test_padded_rows_follow_the_model(env, monkeypatch, change):
         out.append([m._dev[k].cpu().numpy().copy() for k in ("u", m._state_names[0])])
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_inference_mode(env, batch):
+    """Runs under torch.inference_mode(), whose tensors count no writes: the
+    same bits as outside it, also after weights written in place."""
+    fg, autotune = env
+    out = []
+    for inference in (True, False):
+        with torch.inference_mode(inference):
+            m = _model(fg, "MitchellSchaeffer2D", (70, 121), True)
+            m.tracker_sequence.sequence.pop()      # a batch takes no probes
+            m.initialize()
+            autotune._memo[autotune.key(m)] = {"variant": 3, "k": 4, "flat": [1, 4]}
+            runner = fg.TissueBatch([m]) if batch else m
+            m.t_max = 0.995
+            runner.run(initialize=False)
+            m.weights.mul_(0.99)
+            m.t_max = 1.995
+            runner.run(initialize=False)
+            out.append([m.u, m.h] + [np.asarray(t.output)
+                                     for t in m.tracker_sequence.sequence])
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
