@@ -140,7 +140,7 @@ def tune(model, steps=96):
     if model._shape()[1] % 16 and model._pad_ok():
         mir = model._padded()
     if mir is not None:
-        copies = _time_copies(mir, stream)
+        copies = _time_copies(model, mir, stream)
         mir.apply(a)
         for v, k in _TMA:
             try:
@@ -156,7 +156,7 @@ def tune(model, steps=96):
     return {"variant": v, "k": k, "flat": [fv, fk], "ms": times, "steps": steps}
 
 
-def _time_copies(mir, stream, reps=3):
+def _time_copies(model, mir, stream, reps=3):
     """ms of moving a model's state into its padded copies and, unchanged,
     out again."""
     best = float("inf")
@@ -164,8 +164,8 @@ def _time_copies(mir, stream, reps=3):
         e0 = torch.cuda.Event(enable_timing=True)
         e1 = torch.cuda.Event(enable_timing=True)
         e0.record(stream)
-        mir.run_copies(mir.copies_in(), stream.cuda_stream)
-        mir.run_copies(mir.copies_out(), stream.cuda_stream)
+        mir.run_copies(mir.copies_in(model), stream.cuda_stream)
+        mir.run_copies(mir.copies_out(model), stream.cuda_stream)
         e1.record(stream)
         e1.synchronize()
         best = min(best, e0.elapsed_time(e1))

@@ -33,11 +33,12 @@ class _Mirror:
     padded to a multiple of 16 nodes (the row pitch a tensor map needs).
     The batch advances the copies; `copies_in` and `copies_out` list the
     copies that move the model's state between them and the model's own
-    arrays, and `swap` follows the model's u / u_new exchange."""
+    arrays, and `swap` follows the model's u / u_new exchange.  The mirror
+    does not refer to the model, which so is freed when nothing else does."""
 
     def __init__(self, m):
         ni, nj = m._shape()
-        self.model, self.nj = m, nj
+        self.nj = nj
         self.pitch = -(-nj // 16) * 16
         self.weights_src, self.myo_src = m.weights, m._myo_d
         dev = m._device()
@@ -55,19 +56,23 @@ class _Mirror:
         # device address of a tracker's flags -> (flags, padded copy)
         self.act = {}
         self.versions = None
-        self.refresh()
+        self.refresh(m)
+
+    def __reduce__(self):
+        # copies and pickles of what holds a mirror go without it
+        return type(None), ()
 
     def valid_for(self, m):
         """The model's weights and flags are still the tensors that were
         copied."""
-        return (m is self.model and m.weights is self.weights_src and
+        return (m.weights is self.weights_src and
                 m._myo_d is self.myo_src)
 
-    def refresh(self):
+    def refresh(self, m):
         """Copy the weights and flags again where something has been written
         into them since, or may have been: tensors of inference mode do not
         count their writes."""
-        m, versions = self.model, None
+        versions = None
         if not (m.weights.is_inference() or m._myo_d.is_inference()):
             versions = m.weights._version, m._myo_d._version
             if versions == self.versions:
@@ -81,8 +86,9 @@ class _Mirror:
                      self.pitch)], stream)
         self.versions = versions
 
-    def _lat_flags(self):
-        seq = self.model.tracker_sequence
+    @staticmethod
+    def _lat_flags(m):
+        seq = m.tracker_sequence
         if not seq:
             return []
         return [tr._activated for tr in seq.sequence
@@ -97,8 +103,8 @@ class _Mirror:
         return (src.data_ptr(), dst.data_ptr(), ni, self.nj * b, nj_src * b,
                 nj_dst * b)
 
-    def copies_in(self):
-        m, nj, P = self.model, self.nj, self.pitch
+    def copies_in(self, m):
+        nj, P = self.nj, self.pitch
         ni = self.u[0].shape[0]
         out = [self._rows(m._dev["u"], self.u[0], nj, P),
                self._rows(m._dev["u_new"], self.u[1], nj, P)]
@@ -106,7 +112,7 @@ class _Mirror:
             out.append(self._rows(m._dev[name], t, nj, P))
             out.append(self._rows(m._dev[name], tb, nj, P))
         act = {}
-        for f in self._lat_flags():
+        for f in self._lat_flags(m):
             old = self.act.get(f.data_ptr())
             if old is not None and old[0] is f:
                 pad = old[1]
@@ -118,8 +124,8 @@ class _Mirror:
         self.act = act
         return out
 
-    def copies_out(self):
-        m, nj, P = self.model, self.nj, self.pitch
+    def copies_out(self, m):
+        nj, P = self.nj, self.pitch
         out = [self._rows(self.u[0], m._dev["u"], P, nj),
                self._rows(self.u[1], m._dev["u_new"], P, nj)]
         for t, name in zip(self.state, m._state_names):
@@ -198,7 +204,7 @@ class TissueBatch:
             mir = _Mirror(m)
             self._mirrors[id(m)] = mir
         else:
-            mir.refresh()
+            mir.refresh(m)
         return mir
 
     def add(self, model):
@@ -306,7 +312,8 @@ class TissueBatch:
         tma = self.kernel in ("tma", "pairs")
         mirrors = [self._mirror(m) for m in ms] if tma else None
         if tma:
-            _copy_rows([c for mir in mirrors for c in mir.copies_in()], stream)
+            _copy_rows([c for m, mir in zip(ms, mirrors) for c in mir.copies_in(m)],
+                       stream)
         while active:
             limit = min(_MAX_SEGMENT, min(remaining[i] for i in active))
             if self.chunk:
@@ -341,13 +348,13 @@ class TissueBatch:
                 remaining[i] -= n
                 host = tma and (m.command_sequence or m.state_saver)
                 if host:
-                    _copy_rows(mirrors[i].copies_out(), stream)
+                    _copy_rows(mirrors[i].copies_out(m), stream)
                 if m.command_sequence:
                     m.command_sequence.execute_next()
                 if m.state_saver:
                     m.state_saver.save()
                 if host:
-                    _copy_rows(mirrors[i].copies_in(), stream)
+                    _copy_rows(mirrors[i].copies_in(m), stream)
                 if m.check_termination():
                     if m.state_saver:
                         m.state_saver.save()
@@ -356,6 +363,7 @@ class TissueBatch:
                     still.append(i)
             active = still
         if tma:
-            _copy_rows([c for mir in mirrors for c in mir.copies_out()], stream)
+            _copy_rows([c for m, mir in zip(ms, mirrors) for c in mir.copies_out(m)],
+                       stream)
         for m, st in zip(ms, torch.cat([m._status for m in ms]).tolist()):
             m._check_status(st)

@@ -240,6 +240,7 @@ class CardiacModel:
         shape = self._shape()
         dtype = self._torch_dtype()
         self._dev = {}
+        self._pad = None
         u = torch.zeros(shape, dtype=dtype, device=dev)
         self._dev["u"] = u
         self._dev["u_new"] = u.clone()
@@ -289,6 +290,7 @@ class CardiacModel:
         """Myocyte indices, stencil choice and device weights
         (cardiac_model.py:119-128)."""
         tissue = self.cardiac_tissue
+        self._pad = None   # row-padded copies, made when a run asks for them
         tissue.compute_myo_indexes()
         mesh = np.asarray(tissue.mesh)
         myo = mesh == 1
@@ -324,7 +326,6 @@ class CardiacModel:
         self._pack_weights()
         self._weight_rows()
         self._node_order()
-        self._pad = None
 
     def _pad_ok(self):
         """Row-padded copies of the arrays may be kept for the TMA kernels
@@ -347,7 +348,7 @@ class CardiacModel:
             except torch.cuda.OutOfMemoryError:
                 pass
         else:
-            self._pad.refresh()
+            self._pad.refresh(self)
         return self._pad
 
     def _node_order(self):
@@ -667,7 +668,7 @@ class CardiacModel:
         stream = torch.cuda.current_stream().cuda_stream
         pad = self._segment_padding(seg)
         if pad is not None:
-            pad.run_copies(pad.copies_in(), stream)
+            pad.run_copies(pad.copies_in(self), stream)
             variant = seg.args.fused_variant
             pad.apply(seg.args)
             seg.args.fused_variant = variant
@@ -679,7 +680,7 @@ class CardiacModel:
         if pad is not None:
             if seg.n_seg % 2 == 1:
                 pad.swap()
-            pad.run_copies(pad.copies_out(), stream)
+            pad.run_copies(pad.copies_out(self), stream)
         return seg.n_seg
 
     def _segment_padding(self, seg):

@@ -152,3 +152,43 @@ def test_inference_mode(env, batch):
                                      for t in m.tracker_sequence.sequence])
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+def test_padded_copies_end_with_the_model(env):
+    """A model that ran on padded copies is freed with its last reference, its
+    device memory with it, without the cycle collector; clones and a new
+    initialize() start without the copies."""
+    import gc
+    import weakref
+    fg, autotune = env
+    gc.collect()
+    before = torch.cuda.memory_allocated()
+    t = fg.CardiacTissue2D((300, 301))
+    m = fg.AlievPanfilov2D()
+    m.dt, m.dr, m.npfloat, m.cardiac_tissue = 0.01, 0.25, "float32", t
+    m.initialize()
+    autotune._memo[autotune.key(m)] = {"variant": 3, "k": 4, "flat": [1, 4]}
+    held = torch.cuda.memory_allocated()
+    m.t_max = 0.995
+    m.run(initialize=False)
+    padded = m._pad is not None
+    assert padded and torch.cuda.memory_allocated() > held
+    c = m.clone()
+    bare = getattr(c, "_pad", None) is None
+    assert bare
+    c.t_max = m.t_max = 1.995
+    c.run(initialize=False)
+    m.run(initialize=False)
+    assert all(torch.equal(c._dev[k], m._dev[k]) for k in ("u", "v"))
+    del c
+    m.initialize()
+    assert torch.cuda.memory_allocated() <= held
+    m.t_max = 0.995
+    m.run(initialize=False)
+    gc.disable()
+    try:
+        gone = weakref.ref(m)
+        del m
+        assert gone() is None and torch.cuda.memory_allocated() <= before
+    finally:
+        gc.enable()
