@@ -151,6 +151,8 @@ def tune(model, steps=96):
             cost["%d/%d" % (v, k)] = t + copies
     del keep
     best = min(cost, key=cost.get)
+    if best == flat:
+        model._pad = None    # nothing will use the copies
     v, k = (int(x) for x in best.split("/"))
     fv, fk = (int(x) for x in flat.split("/"))
     return {"variant": v, "k": k, "flat": [fv, fk], "ms": times, "steps": steps}

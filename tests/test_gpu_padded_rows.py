@@ -192,3 +192,20 @@ def test_padded_copies_end_with_the_model(env):
         assert gone() is None and torch.cuda.memory_allocated() <= before
     finally:
         gc.enable()
+
+
+def _fake_times(monkeypatch, autotune, cpasync, tma, copies):
+    """A tuner that finds these ms for 96 steps and for the copies."""
+    monkeypatch.setattr(autotune, "_time_candidate",
+                        lambda model, a, v, k, steps, stream: tma if v in (3, 4) else cpasync)
+    monkeypatch.setattr(autotune, "_time_copies", lambda *a: copies)
+
+
+def test_copies_are_dropped_where_they_lose(env, monkeypatch):
+    fg, autotune = env
+    m = _model(fg, "AlievPanfilov2D", (60, 77), False)
+    m.initialize()
+    _fake_times(monkeypatch, autotune, 1.0, 0.8, 0.3)
+    m.t_max = 1.195
+    m.run(initialize=False)
+    assert m._pad is None and m._fused_choice == (1, 2)
