@@ -98,7 +98,10 @@ def _time_candidate(model, args, variant, k, steps, stream, reps=3):
 
 def tune(model, steps=96):
     """Time every fused candidate for `model` (initialised, fused form) on
-    scratch copies of its arrays; returns {"variant": v, "k": k, "ms": {...}}.
+    scratch copies of its arrays; returns {"variant": v, "k": k, "ms": {...}}
+    and, where padded copies were timed, "flat" (the best choice on the
+    model's own arrays) and "pad_from" (the steps in which the copies in and
+    out are made up for).
     """
     saved = model.autotune
     model.autotune = False
@@ -136,6 +139,7 @@ def tune(model, steps=96):
     # 2.7 against 2.0)
     flat = min(times, key=times.get)
     cost = dict(times)
+    pad_from = 0
     mir = None
     if model._shape()[1] % 16 and model._pad_ok():
         mir = model._padded()
@@ -151,11 +155,15 @@ def tune(model, steps=96):
             cost["%d/%d" % (v, k)] = t + copies
     del keep
     best = min(cost, key=cost.get)
-    if best == flat:
-        model._pad = None    # nothing will use the copies
+    if mir is not None:
+        if best == flat:
+            model._pad = None    # nothing will use the copies
+        else:
+            pad_from = math.ceil(copies * steps / (times[flat] - times[best]))
     v, k = (int(x) for x in best.split("/"))
     fv, fk = (int(x) for x in flat.split("/"))
-    return {"variant": v, "k": k, "flat": [fv, fk], "ms": times, "steps": steps}
+    return {"variant": v, "k": k, "flat": [fv, fk], "pad_from": pad_from,
+            "ms": times, "steps": steps}
 
 
 def _time_copies(model, mir, stream, reps=3):
@@ -174,30 +182,34 @@ def _time_copies(model, mir, stream, reps=3):
     return best
 
 
-def choose_flat(model):
-    """The fastest candidate on the model's own arrays (rows of any length)."""
-    choose(model)
-    with _lock:
-        r = _memo[key(model)]
-    return tuple(r.get("flat") or (r["variant"], r["k"]))
+def flat(model):
+    """((fused_variant, fused_k), steps): the fastest candidate on the model's
+    own arrays (rows of any length), and the number of steps from which a
+    chosen TMA kernel on padded copies is faster (0: not measured)."""
+    r = _entry(model)
+    return tuple(r.get("flat") or (r["variant"], r["k"])), r.get("pad_from", 0)
 
 
 def choose(model):
     """(fused_variant, fused_k) for `model`: from the cache, else tuned now
     and cached."""
+    r = _entry(model)
+    return r["variant"], r["k"]
+
+
+def _entry(model):
     kk = key(model)
     with _lock:
         if kk in _memo:
-            r = _memo[kk]
-            return r["variant"], r["k"]
+            return _memo[kk]
         table = _load()
         if kk in table:
             _memo[kk] = table[kk]
-            return table[kk]["variant"], table[kk]["k"]
+            return table[kk]
     r = tune(model)
     with _lock:
         _memo[kk] = r
         table = _load()
         table[kk] = r
         _store(table)
-    return r["variant"], r["k"]
+    return r

@@ -33,7 +33,8 @@ _NP = {"float64": np.float64, "float32": np.float32}
 _MAX_SEGMENT = 1 << 20
 # steps of a segment from which rows of no multiple of 16 nodes run on padded
 # copies, where the tuner, which counts the copies in and out against 96
-# steps, found that faster
+# steps, found that faster, and from the steps at which it found the copies
+# made up for
 _PAD_MIN_STEPS = 64
 
 
@@ -692,12 +693,13 @@ class CardiacModel:
         if (a.form != _ffi.FORM_FUSED or a.weights_packed or self.fused_k or
                 self.fused_variant or a.fused_variant not in (3, 4)):
             return None
-        if self._pad_ok() and seg.n_seg >= _PAD_MIN_STEPS:
+        from . import autotune
+        flat, pad_from = autotune.flat(self)
+        if self._pad_ok() and seg.n_seg >= max(_PAD_MIN_STEPS, pad_from):
             pad = self._padded()
             if pad is not None:
                 return pad
-        from . import autotune
-        a.fused_variant, a.fused_k = autotune.choose_flat(self)
+        a.fused_variant, a.fused_k = flat
         return None
 
     def _bare_args(self, tune=True):

@@ -209,3 +209,17 @@ def test_copies_are_dropped_where_they_lose(env, monkeypatch):
     m.t_max = 1.195
     m.run(initialize=False)
     assert m._pad is None and m._fused_choice == (1, 2)
+
+
+def test_copies_from_the_measured_steps(env, monkeypatch):
+    """0.5 ms saved in 96 steps make up for copies of 0.4 ms in 77 steps."""
+    fg, autotune = env
+    m = _model(fg, "AlievPanfilov2D", (60, 77), False)
+    m.initialize()
+    _fake_times(monkeypatch, autotune, 1.5, 1.0, 0.4)
+    assert autotune.choose(m) == (3, 2) and autotune.flat(m) == ((1, 2), 77)
+    for steps, padded in ((76, False), (77, True)):
+        m._pad = None
+        m.t_max = m.t + (steps - 0.5) * m.dt
+        m.run(initialize=False)
+        assert (m._pad is not None) == padded
