@@ -75,7 +75,8 @@ def key(model):
     parts = [name, type(model).__name__, str(model.stencil.kind),
              "%dD" % len(shape), "2^%d" % int(math.log2(max(n, 1)))]
     if len(shape) == 2 and shape[1] % 16:
-        parts.append("ragged")   # the TMA kernels run on padded copies
+        # the TMA kernels run on padded copies, where the model may keep any
+        parts.append("ragged" if model._pad_ok() else "ragged flat")
     return "|".join(parts)
 
 
@@ -207,6 +208,7 @@ def _entry(model):
             _memo[kk] = table[kk]
             return table[kk]
     r = tune(model)
+    kk = key(model)    # a model that found no room for copies has another
     with _lock:
         _memo[kk] = r
         table = _load()

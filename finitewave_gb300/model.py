@@ -292,6 +292,7 @@ class CardiacModel:
         (cardiac_model.py:119-128)."""
         tissue = self.cardiac_tissue
         self._pad = None   # row-padded copies, made when a run asks for them
+        self._pad_room = True
         tissue.compute_myo_indexes()
         mesh = np.asarray(tissue.mesh)
         myo = mesh == 1
@@ -334,6 +335,7 @@ class CardiacModel:
         counted its own arrays)."""
         shape = self._shape()
         return (getattr(self, "pad_rows", True) and
+                getattr(self, "_pad_room", True) and
                 len(shape) == 2 and shape[1] % 16 != 0 and
                 self.stencil.kind in (_ffi.ISO5, _ffi.ANISO9) and
                 self._model_id in self._FUSED_MODELS)
@@ -347,7 +349,7 @@ class CardiacModel:
             try:
                 self._pad = _Mirror(self)
             except torch.cuda.OutOfMemoryError:
-                pass
+                self._pad_room = False
         else:
             self._pad.refresh(self)
         return self._pad

@@ -223,3 +223,29 @@ def test_copies_from_the_measured_steps(env, monkeypatch):
         m.t_max = m.t + (steps - 0.5) * m.dt
         m.run(initialize=False)
         assert (m._pad is not None) == padded
+
+
+def test_choice_without_copies_is_its_own(env, monkeypatch, tmp_path):
+    """What a model that may not, or cannot, keep copies was given is not
+    what the next model with copies gets."""
+    fg, autotune = env
+    from finitewave_gb300 import batch
+    _fake_times(monkeypatch, autotune, 1.5, 1.0, 0.1)
+
+    def no_room(model):
+        raise torch.cuda.OutOfMemoryError("no room")
+    for why in ("pad_rows", "no room"):
+        autotune._memo.clear()
+        monkeypatch.setenv("FWGPU_AUTOTUNE_CACHE", str(tmp_path / (why + ".json")))
+        m = _model(fg, "AlievPanfilov2D", (60, 77), False)
+        m.initialize()
+        with monkeypatch.context() as mp:
+            if why == "pad_rows":
+                m.pad_rows = False
+            else:
+                mp.setattr(batch, "_Mirror", no_room)
+            assert autotune.choose(m) == (1, 2)
+            assert autotune.choose(m) == (1, 2)
+        m = _model(fg, "AlievPanfilov2D", (60, 77), False)
+        m.initialize()
+        assert autotune.choose(m) == (3, 2), why
