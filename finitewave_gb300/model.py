@@ -357,19 +357,31 @@ class CardiacModel:
     def _node_order(self):
         """The nodes with the myocytes first (fw_step_args.node_list), for
         the plain steps that run one thread per myocyte: float64 and the
-        detailed models."""
+        detailed models.  (Not from flags made in inference mode, whose
+        writes are not counted: `_node_list` could not follow them.)"""
         self._nodes = None
         if (self._precision() == _ffi.F32 and
                 self._model_id not in self._DETAILED_MODELS):
             return
         n = self._myo_d.numel()
-        if n < 1 << 31:
+        if n < 1 << 31 and not self._myo_d.is_inference():
             dev = self._myo_d.device
             self._nodes = torch.empty(n, dtype=torch.int32, device=dev)
             scratch = torch.empty(n // 4096 + 2, dtype=torch.int32, device=dev)
             _ffi.call("fw_node_list", self._myo_d.data_ptr(), n,
                       self._nodes.data_ptr(), scratch.data_ptr(),
                       torch.cuda.current_stream().cuda_stream)
+            self._nodes_src = self._myo_d, self._myo_d._version
+
+    def _node_list(self):
+        """The node order of the myocyte flags as they are: made again where
+        the flags were replaced or written to."""
+        if getattr(self, "_nodes", None) is not None:
+            src, version = self._nodes_src
+            if src is not self._myo_d or src._version != version:
+                self._n_myo = int(torch.count_nonzero(self._myo_d))
+                self._node_order()
+        return getattr(self, "_nodes", None)
 
     def _weight_rows(self, force=False):
         """FW_STENCIL_ANISO19_XY steps read the eleven weight planes 0-8,
@@ -724,7 +736,7 @@ class CardiacModel:
             if self._wrows is not None and a.stencil == _ffi.ANISO19_XY:
                 a.weight_rows = self._wrows.data_ptr()
                 a.weight_row_index = self._widx.data_ptr()
-        nodes = getattr(self, "_nodes", None)
+        nodes = self._node_list()
         if nodes is not None:
             a.node_list = nodes.data_ptr()
             a.n_list_myo = self._n_myo

@@ -114,3 +114,30 @@ def test_listed_activation_at_non_myocytes(fg, cls, npfloat, shape, start, step)
         out.append([np.asarray(tr.output) for tr in trs.sequence])
     for a, b in zip(*out):
         assert np.array_equal(a, b) and (a >= 0).any()
+
+
+@pytest.mark.parametrize("cls,npfloat", [("AlievPanfilov2D", "float64"), ("TP062D", "float32")])
+@pytest.mark.parametrize("how", ["in place", "replaced", "inference"])
+def test_node_list_follows_the_flags(fg, cls, npfloat, how):
+    """Myocyte flags cleared and set between two runs: the steps are those of
+    grid order, on a grid that is large enough for the list."""
+    out = []
+    for listed in (True, False):
+        with torch.inference_mode(how == "inference"):
+            m, trs = _model(fg, getattr(fg, cls), npfloat, (150, 161), False)
+            m.initialize()
+            if not listed:
+                m._nodes = None
+            m.run(initialize=False)
+            myo = m._myo_d if how != "replaced" else m._myo_d.clone()
+            myo[20:60] = 0
+            inner = myo[70:90, 1:-1]
+            inner.copy_((torch.arange(inner.numel(), device=myo.device) % 3 > 0)
+                        .to(torch.int8).reshape(inner.shape))
+            m._myo_d = myo
+            m.t_max = 0.4
+            m.run(initialize=False)
+            out.append([getattr(m, n) for n in ["u", "u_new"] + list(m._state_names)] +
+                       [t.output for t in trs])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
