@@ -269,10 +269,10 @@ class SimulationServer:
             if status is not None else None
         keep.append(status)
         r._keep = keep
-        m._dev = {}
-        m.weights = None
-        m._wpack = None
-        m._mesh_d = m._myo_d = None
+        m._dev, m._stateb = {}, {}
+        m.weights = m._wpack = m._pad = None
+        m._wrows = m._wrows_src = m._widx = None
+        m._mesh_d = m._myo_d = m._nodes = m._nodes_src = None
         return ops.record(self._copy)
 
     def _finish_release(self, r):

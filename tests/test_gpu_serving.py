@@ -5,6 +5,7 @@ tracker outputs equal those of the same model run alone; requests on their
 own streams run on the device at the same time (their device spans
 overlap) and still give each request's results alone, bit for bit."""
 import copy
+import gc
 
 import numpy as np
 import pytest
@@ -134,3 +135,31 @@ def test_requests_overlap_on_device(env):
         assert r.steps == 60
         assert np.array_equal(at.output, act), r.name
         assert r.snapshot() is not None
+
+
+def _sheet(fg, cls, npfloat):
+    t = fg.CardiacTissue2D((700, 703))
+    t.fibers = np.zeros((700, 703, 2))
+    t.fibers[..., 0] = 1
+    m = getattr(fg, cls)()
+    m.dt, m.dr, m.t_max, m.npfloat, m.cardiac_tissue = 0.01, 0.25, 0.05, npfloat, t
+    return m
+
+
+def _requested():
+    gc.collect()
+    return torch.cuda.memory_stats()["requested_bytes.all.current"]
+
+
+SHEETS = [("AlievPanfilov2D", "float64"), ("TP062D", "float32"), ("AlievPanfilov2D", "float32")]
+
+
+@pytest.mark.parametrize("cls,npfloat", SHEETS)
+def test_finished_request_holds_nothing(env, cls, npfloat):
+    """A finished request holds no device memory but a few words of status
+    and flags."""
+    fg, _ = env
+    before = _requested()
+    r = fg.Request(_sheet(fg, cls, npfloat))
+    assert fg.SimulationServer().serve([r], realtime=False) == [r]
+    assert _requested() - before <= 1024
