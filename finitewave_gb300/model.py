@@ -354,18 +354,20 @@ class CardiacModel:
             self._pad.refresh(self)
         return self._pad
 
+    def _has_node_order(self):
+        """Whether the model's plain steps run from the node list."""
+        return (int(np.prod(self._shape())) < 1 << 31 and
+                (self._precision() == _ffi.F64 or
+                 self._model_id in self._DETAILED_MODELS))
+
     def _node_order(self):
         """The nodes with the myocytes first (fw_step_args.node_list), for
         the plain steps that run one thread per myocyte: float64 and the
         detailed models.  (Not from flags made in inference mode, whose
         writes are not counted: `_node_list` could not follow them.)"""
         self._nodes = None
-        if (self._precision() == _ffi.F32 and
-                self._model_id not in self._DETAILED_MODELS):
-            return
-        n = self._myo_d.numel()
-        if n < 1 << 31 and not self._myo_d.is_inference():
-            dev = self._myo_d.device
+        if self._has_node_order() and not self._myo_d.is_inference():
+            n, dev = self._myo_d.numel(), self._myo_d.device
             self._nodes = torch.empty(n, dtype=torch.int32, device=dev)
             scratch = torch.empty(n // 4096 + 2, dtype=torch.int32, device=dev)
             _ffi.call("fw_node_list", self._myo_d.data_ptr(), n,

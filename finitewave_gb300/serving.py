@@ -4,9 +4,10 @@ The reference runs one simulation per ``model.run()`` call.  The server
 takes simulation requests -- configured models of any family, 2D or 3D, each
 with its own tissue, stimuli, trackers and ``t_max`` -- as they arrive, and
 
-* admits them first come, first served while the device footprint of the
+* admits them first come, first served while the device bytes of the
   admitted requests (state, weights, mesh and tracker buffers: bytes per node
-  x nodes, `device_footprint`) stays within an HBM budget;
+  x nodes, `device_footprint`; and the order of the nodes that listed steps
+  read) stay within an HBM budget;
 * prepares an admitted request (``initialize()``: host mesh work, uploads,
   the weight build) on a worker thread and on the request's own CUDA stream,
   so the loop keeps issuing work for the running requests meanwhile;
@@ -38,6 +39,7 @@ import numpy as np
 import torch
 
 from . import _ffi
+from .model import CardiacModel
 
 _STATE_BYTES = {_ffi.F64: 8, _ffi.F32: 4}
 
@@ -45,7 +47,9 @@ _STATE_BYTES = {_ffi.F64: 8, _ffi.F32: 4}
 def device_footprint(model):
     """Device bytes a model will hold once initialised: u and u_new, the
     state variables, the stencil weights (and the packed copy of the fused
-    form), mesh and myocyte flags, and its trackers' buffers."""
+    form), mesh and myocyte flags, and its trackers' buffers.  (Not the
+    4 bytes a node of the node order of float64 and detailed models, which
+    the admission adds.)"""
     shape = tuple(np.asarray(model.cardiac_tissue.mesh).shape)
     n = int(np.prod(shape))
     prec = model._precision()
@@ -68,6 +72,15 @@ def device_footprint(model):
         elif name.startswith("LocalActivationTime"):
             per_node += 1 + 4 + 4 * int(getattr(tr, "capacity", 16))
     return n * per_node
+
+
+def _admission_bytes(model):
+    """What an admitted request counts against the budget: its footprint and
+    its node order."""
+    n = device_footprint(model)
+    if isinstance(model, CardiacModel) and model._has_node_order():
+        n += 4 * int(np.prod(model._shape()))
+    return n
 
 
 class Request:
@@ -315,7 +328,7 @@ class SimulationServer:
                 t = now()
                 while pending and (not realtime or pending[0].arrival <= t):
                     r = pending.popleft()
-                    r.footprint = device_footprint(r.model)
+                    r.footprint = _admission_bytes(r.model)
                     if r.footprint > budget:
                         self.rejected.append(r)
                     else:

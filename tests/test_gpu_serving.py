@@ -163,3 +163,19 @@ def test_finished_request_holds_nothing(env, cls, npfloat):
     r = fg.Request(_sheet(fg, cls, npfloat))
     assert fg.SimulationServer().serve([r], realtime=False) == [r]
     assert _requested() - before <= 1024
+
+
+@pytest.mark.parametrize("cls,npfloat", SHEETS)
+def test_admission_covers_what_a_request_holds(env, cls, npfloat):
+    """The bytes counted against the budget are at least those initialize()
+    asks for (without the fused form's second state buffers, which are not in
+    the estimate, and a few words of status and flags)."""
+    fg, _ = env
+    before = _requested()
+    m = _sheet(fg, cls, npfloat)
+    m.initialize()
+    held = _requested() - before
+    second = sum(t.numel() * t.element_size() for t in m._stateb.values())
+    r = fg.Request(_sheet(fg, cls, npfloat))
+    assert fg.SimulationServer().serve([r], realtime=False) == [r]
+    assert held - second <= r.footprint + 1024

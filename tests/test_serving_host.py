@@ -175,3 +175,16 @@ def test_stats(fake_cuda):
     assert st["myocyte_steps"] == 10 * sum(2 + i for i in range(5))
     empty = serving.SimulationServer(hbm_budget=1).stats()
     assert empty == {"completed": 0, "rejected": 0}
+
+
+def test_admission_counts_the_node_order():
+    """Float64 and detailed models keep 4 bytes a node more than
+    device_footprint; float32 phenomenological ones do not."""
+    import numpy as np
+    import finitewave_gb300 as fg
+    for cls, prec, extra in (("AlievPanfilov2D", "float64", 4), ("TP062D", "float32", 4),
+                             ("TP062D", "float64", 4), ("AlievPanfilov2D", "float32", 0)):
+        m = getattr(fg, cls)()
+        m.npfloat = prec
+        m.cardiac_tissue = fg.CardiacTissue2D((30, 40))
+        assert serving._admission_bytes(m) == fg.device_footprint(m) + extra * 1200
