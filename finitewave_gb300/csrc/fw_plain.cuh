@@ -103,9 +103,12 @@ struct StepK {
     T dt;
     int64_t n, si, sj;
     // nodes in list order, myocytes first (NULL: every node in grid order);
-    // n_run threads' worth of them are visited, the first n_myo step
+    // the first n_myo of them step.  The launch's first `rest` CTAs show the
+    // other nodes to the local activation trackers and, with rest_at, to the
+    // activation trackers
     const int32_t *list;
-    int32_t n_run, n_myo;
+    int32_t n_myo, rest;
+    bool rest_at;
     int64_t step;
     int32_t n_at, n_lat;
     AtK<T> at[FW_MAX_AT];
@@ -160,6 +163,47 @@ __device__ __forceinline__ void track(const StepK<M, T> &k, int64_t p, T uc)
     }
 }
 
+// The trackers at the nodes that do not step, which follow the myocytes in
+// the list: kRestNodes nodes a thread and round, whose loads are all under
+// way before the first is used.
+constexpr int kRestNodes = 4;
+template <int N, class M, class T>
+__device__ __forceinline__ void rest_nodes(const StepK<M, T> &k, int64_t t0)
+{
+    int64_t p[N];
+    T u[N];
+    bool look[N];   // a tracker has something to record
+#pragma unroll
+    for (int q = 0; q < N; ++q) p[q] = k.list[t0 + q * (int64_t)blockDim.x];
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+        u[q] = k.u[p[q]];
+        look[q] = k.rest_at;
+    }
+    for (int l = 0; l < k.n_lat; ++l) {
+        uint8_t act[N];
+#pragma unroll
+        for (int q = 0; q < N; ++q) act[q] = k.lat[l].activated[p[q]];
+#pragma unroll
+        for (int q = 0; q < N; ++q)
+            look[q] |= act[q] ? u[q] < k.lat[l].thr : u[q] >= k.lat[l].thr;
+    }
+#pragma unroll
+    for (int q = 0; q < N; ++q)
+        if (look[q]) track(k, p[q], u[q]);
+}
+// part `part` of `parts` of them
+template <class M, class T>
+__device__ __forceinline__ void track_rest(const StepK<M, T> &k, int part, int parts)
+{
+    const int64_t round = (int64_t)blockDim.x * kRestNodes;
+    int64_t t0 = k.n_myo + part * round + threadIdx.x;
+    for (; t0 + (kRestNodes - 1) * (int64_t)blockDim.x < k.n; t0 += parts * round)
+        rest_nodes<kRestNodes>(k, t0);
+    for (int q = 0; q < kRestNodes && t0 < k.n; ++q, t0 += blockDim.x)
+        rest_nodes<1>(k, t0);
+}
+
 // Minimum resident CTAs per SM asked of the compiler for the float32
 // k_step: models may set M::kMinBlocksF32 (the detailed models trade
 // registers for the occupancy their memory latency needs); 1 otherwise.
@@ -211,6 +255,16 @@ constexpr int step_threads()
     return sizeof(T) == 8 ? 32 : kThreads;
 }
 
+// Threads that show the other nodes to the trackers (track_rest), as CTAs
+// before those that step: 512 an SM, so that myocytes step beside them while
+// their loads are under way.  Us a step with one local activation tracker, in
+// grid order, with the other nodes one a thread behind the myocytes, and so:
+// TP06 float32 236^3 shell (7 % myocytes) 185, 211, 132, 192^3 shell (16 %)
+// 132, 133, 89, Aliev-Panfilov float64 192^3 shell 327, 300, 139, 600 x 601
+// (79 %) 41.4, 28.8, 29.0, TP06 float32 600 x 601 18.9, 10.7, 10.5; with 256
+// an SM 186, 110, 139, 29.0, 10.5, with 1024 131, 94, 139, 29.0, 10.5.
+constexpr int kRestThreads = 152 * 512;
+
 // CTAs of a step.  Listed steps run one node per thread; the others, bound
 // by memory, loop over the grid with the resident CTAs.
 template <class M, class T>
@@ -225,7 +279,7 @@ __global__ void __launch_bounds__(step_threads<T>(), (MinBlocks<M, T>::value))
 {
     const Params<T, M::NP + M::ND> P = load_params<T, M::NP + M::ND>(k.params);
     const T dt = k.dt;
-    const int64_t n = LIST ? (int64_t)k.n_run : k.n;
+    const int64_t n = LIST ? (int64_t)k.n_myo : k.n;
     // Steps of one call follow one another with programmatic serialisation:
     // the next one's CTAs take their places, read their parameters and wait
     // here while this one's last CTAs run.  A listed float64 step lets them
@@ -245,13 +299,21 @@ __global__ void __launch_bounds__(step_threads<T>(), (MinBlocks<M, T>::value))
                 k.up[a].out[c] = (double)k.u[k.up[a].cells[c]];
         return;
     }
-    const int64_t stride = (int64_t)(gridDim.x - (k.n_up ? 1 : 0)) * blockDim.x;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
-         t += stride) {
+    int cta = (int)blockIdx.x, ctas = (int)gridDim.x - (k.n_up ? 1 : 0);
+    if constexpr (LIST) {
+        if (cta < k.rest) {
+            track_rest(k, cta, k.rest);
+            return;
+        }
+        cta -= k.rest;
+        ctas -= k.rest;
+    }
+    const int64_t stride = (int64_t)ctas * blockDim.x;
+    for (int64_t t = cta * (int64_t)blockDim.x + threadIdx.x; t < n; t += stride) {
         const int64_t p = LIST ? (int64_t)k.list[t] : t;
         T uc = k.u[p];
         if (k.n_at | k.n_lat) track(k, p, uc);
-        if (LIST ? t >= k.n_myo : !k.myo[p]) continue;
+        if (!LIST && !k.myo[p]) continue;
         T un;
         if constexpr (ST == FW_STENCIL_ANISO19_XY) {
             if (k.wrow)
@@ -648,8 +710,12 @@ int run_plain(const fw_step_args *a, int64_t n_begin, int64_t n_steps,
     const int threads = sizeof(T) == 4 && listed ? kListThreadsF32 : step_threads<T>();
     k.list = listed ? a->node_list : nullptr;
     k.n_myo = (int32_t)a->n_list_myo;
-    const int blocks_all = grid_for(g.n, threads, step_blocks<M, T>());
-    const int blocks_myo = grid_for(a->n_list_myo, threads, step_blocks<M, T>());
+    const int blocks = !listed         ? grid_for(g.n, threads, step_blocks<M, T>())
+                       : a->n_list_myo ? grid_for(a->n_list_myo, threads,
+                                                  step_blocks<M, T>())
+                                       : 0;
+    const int blocks_rest = grid_for(g.n - a->n_list_myo, threads * kRestNodes,
+                                     kRestThreads / threads);
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     cudaLaunchConfig_t cfg = {};
@@ -716,19 +782,18 @@ int run_plain(const fw_step_args *a, int64_t n_begin, int64_t n_steps,
         // the trackers also watch the nodes that do not step: the local
         // activation ones each time (a node may differ between the buffers
         // and cross back), the others, which record the first time only, once
-        // for each buffer and stimulus.  TP06 float32 on a 236^3 shell with
-        // 7 % myocytes: 186 us a step with all nodes visited each time,
-        // 90 so (163 in grid order, before there was a list).
-        const bool all = k.n_lat || (active & ~seen[s & 1]) || !listed;
-        if (all) seen[s & 1] |= active;
-        k.n_run = all ? (int32_t)(listed ? g.n : 0) : k.n_myo;
+        // for each buffer and stimulus.
+        k.rest_at = (active & ~seen[s & 1]) != 0;
+        k.rest = listed && (k.n_lat || k.rest_at) ? blocks_rest : 0;
+        if (k.rest_at) seen[s & 1] |= active;
+        const int ctas = blocks + k.rest + (k.n_up ? 1 : 0);
         attr.val.programmaticStreamSerializationAllowed = s > 0;
-        cfg.gridDim = dim3((unsigned)((all ? blocks_all : blocks_myo) + (k.n_up ? 1 : 0)));
+        cfg.gridDim = dim3((unsigned)ctas);
         auto kern = k_step<M, ST, T, false>;
         if constexpr (UseList<M, T>::value) {
             if (listed) kern = k_step<M, ST, T, true>;
         }
-        if (!listed || k.n_run > 0 || k.n_up) {
+        if (ctas) {
             FW_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, k));
             FW_CHECK_LAUNCH("k_step");
         }

@@ -141,3 +141,42 @@ def test_node_list_follows_the_flags(fg, cls, npfloat, how):
                        [t.output for t in trs])
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("npfloat", ["float64", "float32"])
+@pytest.mark.parametrize("shape,share", [((83, 81, 79), 0.05), ((27, 28, 26), 0.0),
+                                         ((28, 27, 26), 0.999), ((30, 27, 25), 0.8)])
+def test_listed_local_activation_at_non_myocytes(fg, npfloat, shape, share):
+    """Local activation trackers at nodes that do not step, few and many (more
+    than one round of 152 x 512 threads of four), with values on either side
+    of the thresholds in each potential buffer: as in grid order."""
+    out = []
+    for listed in (True, False):
+        gen = np.random.default_rng(7)
+        t = fg.CardiacTissue3D(shape)
+        t.mesh = np.where(gen.random(shape) < share, 1, 2).astype(np.int8)
+        m = fg.TP063D()
+        m.dt, m.dr, m.npfloat, m.cardiac_tissue, m.t_max = 0.01, 0.25, npfloat, t, 0.085
+        trs = fg.TrackerSequence()
+        for cls, thr in ((fg.LocalActivationTime3DTracker, 0.5),
+                         (fg.LocalActivationTime3DTracker, 0.2),
+                         (fg.ActivationTime3DTracker, 0.7)):
+            tr = cls()
+            tr.threshold = thr
+            trs.add_tracker(tr)
+        trs.sequence[1].start_time, trs.sequence[1].step = 0.03, 3
+        m.tracker_sequence = trs
+        m.initialize()
+        for name in ("u", "u_new"):
+            u = m._dev[name]
+            r = torch.as_tensor(gen.random(shape), device=u.device, dtype=u.dtype)
+            u.copy_(torch.where(m._myo_d.reshape(shape) == 0, r, u))
+        if not listed:
+            m._nodes = None
+        m.run(initialize=False)
+        out.append([tr._steps.cpu().numpy() for tr in trs.sequence[:2]] +
+                   [tr._count.cpu().numpy() for tr in trs.sequence[:2]] +
+                   [np.asarray(trs.sequence[2].output), m.u])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+    assert (out[0][2] > 1).any()   # nodes that cross again and again
