@@ -214,9 +214,11 @@ struct ModelAP {
 // The fused kernels' float32 updates of the next models (update_fused): the
 // same expressions, each quotient by a parameter taken as a product with the
 // parameter's reciprocal, which the compiler forms once a tile.  A quotient
-// under --prec-div=false is that reciprocal and product, bit for bit while
-// the divisor is within 2^-126 .. 2^126, but costs six instructions every
-// time; the product stays out of any fused multiply-add, as the quotient did.
+// under --prec-div=false is that reciprocal and product (while the divisor is
+// within 2^-126 .. 2^126), but costs six instructions every time.  The
+// product is a plain one, which the compiler contracts with the sum it enters
+// where it contracted the quotient's: the bits are the quotients' (kept out
+// of the contraction they would not be), and the same in every kernel.
 __device__ __forceinline__ float over(float a, float b)
 {
     return a * dm::rcp(b);
