@@ -356,6 +356,16 @@ __device__ __forceinline__ float ex_by(float x, double, float, float c) { return
     fw::dm::ex_by(X, (double)(S), (float)(256 * fw::dm::kLog2e * (S)), \
                   (float)(fw::dm::kLog2e * (S)))
 
+// The same, float32 rounding x s before it is scaled for ex2, which has no
+// rounding of log2(e) s for an error of every argument: one product more.
+__device__ __forceinline__ double ex_of(double x, double s, float sf, float)
+{
+    return ex_scaled(x, s, sf);
+}
+__device__ __forceinline__ float ex_of(float x, double, float, float s) { return ex(x * s); }
+#define FW_EX_OF(X, S) \
+    fw::dm::ex_of(X, (double)(S), (float)(256 * fw::dm::kLog2e * (S)), (float)(S))
+
 // What a step of dt does to a gate of the given rate, and the gate's next
 // value inf - (inf - x) e^(-dt rate).  ndt is -dt in float64, where the
 // exponential less one is formed without rounding the exponential first and

@@ -263,8 +263,8 @@ struct ModelTP06 {
     // and appended to them (a dozen divisions, a logarithm and a square root
     // per node and step otherwise).
     enum {
-        d_pkn = NP, d_gkr, d_kz, d_cal, d_kw, d_ncx, d_nao3, d_nak, d_naf,
-        d_ssf, d_vcss, d_vsrss, d_ec2, d_kup2, d_dsr, d_lim, d_end
+        d_pkn = NP, d_gkr, d_kz, d_cal, d_kw, d_ncx, d_nao3, d_nak, d_naf, d_icf,
+        d_ssf, d_vcss, d_vsrss, d_ec2, d_kup2, d_mec, d_lim, d_end
     };
     static constexpr int ND = d_end - NP;
     static void derive(const double *p, double dt, double *q)
@@ -282,12 +282,13 @@ struct ModelTP06 {
         q[d_nao3] = nao3 * 2.5;
         q[d_nak] = p[knak] * (p[ko] / (p[ko] + p[KmK]));
         q[d_naf] = dt * inverseVcF * p[CAPACITANCE];
+        q[d_icf] = (double)(1.0f / ((float)p[Vc] * (float)p[F]));
         q[d_ssf] = p[CAPACITANCE] / (2.0 * p[Vss] * p[F]);
         q[d_vcss] = p[Vc] / p[Vss];
         q[d_vsrss] = p[Vsr] / p[Vss];
         q[d_ec2] = p[EC] * p[EC];
         q[d_kup2] = p[Kup] * p[Kup];
-        q[d_dsr] = p[maxsr] - p[minsr];
+        q[d_mec] = p[maxsr] * p[EC] * p[EC];
         // exponents z = (u - 15) d_kz, n u d_kw, (n - 1) u d_kw and u d_kw,
         // d_kw = d_kz / 2
         const double n = fmax(fmax(fabs(p[n_]), fabs(p[n_] - 1.0)), 2.0);
@@ -327,9 +328,12 @@ struct ModelTP06 {
     // instead of 2306 float64 instructions a node (192 x 190 nodes: 60 against
     // 150 us a step, the float64 pipe 83 % busy in both) and 700 instead of
     // 1070 float32 ones (256 x 256 x 40: 104 against 107 us, then bound by the
-    // latency of its loads).  Against 113-bit arithmetic every variable is as
-    // close or closer; the subspace calcium, whose quadratic loses four digits
-    // in the reference's form, 400 times.
+    // latency of its loads).  Against 113-bit arithmetic, one step from states of
+    // a tissue in activity, the rms error of every variable is at most that of
+    // the reference's order (float64 m 5.25e-17 of itself against 5.46e-17,
+    // oo 1.19e-16 against 1.29e-16, xs 4.7e-17 against 1.5e-16; float32 Ki
+    // 9.71e-15 against 9.72e-15); the subspace calcium, whose quadratic loses
+    // four digits in the reference's form, is 56 times closer.
     template <class T>
     __device__ static __forceinline__ T update_in_range(T u, T un, St<T> &x,
                                                         const Params<T, NP + ND> &P,
@@ -352,11 +356,15 @@ struct ModelTP06 {
         // calc_ina
         T ina;
         {
-            const T a = FW_AT(g5, -60.0, 5.0, 162754.79141900392), b = FW_AT(g5, -35.0, 5.0, 1096.6331584284585);
-            const T c = FW_EX(u - (T)50.0, 1 / 200.0);
-            const T rate_m = (c1 + a) * (c1 + b) * (c1 + c) *
-                             rcp((T)0.1 * a * ((T)2.0 + b + c));
-            const T rm = rcp_near(c1 + FW_EX(u + (T)56.86, -1 / 9.03));
+            // a step is of the size of tau_m, so an error of rate_m is one of
+            // m: no exponential common to numerator and denominator here
+            const T da = c1 + FW_EX_OF(u + (T)60.0, -1 / 5.0);
+            T eb;
+            if constexpr (sizeof(T) == 8) eb = FW_AT(g5, -35.0, 5.0, 1096.6331584284585);
+            else eb = FW_EX_OF(u + (T)35.0, 1 / 5.0);
+            const T db = c1 + eb, dc = c1 + FW_EX_OF(u - (T)50.0, 1 / 200.0);
+            const T rate_m = da * (db * dc) * rcp((T)0.1 * (db + dc));
+            const T em = c1 + FW_EX(u + (T)56.86, -1 / 9.03);
             T rate_h, rate_j;
             if (u >= (T)(-40.0)) {
                 rate_h = (T)(0.77 / 0.13) * rcp(c1 + FW_EX(u + (T)10.66, -1 / 11.1));
@@ -373,7 +381,7 @@ struct ModelTP06 {
             }
             const T rh = rcp_near(c1 + FW_EX(u + (T)71.55, 1 / 7.43));
             const T h_inf = rh * rh;
-            x.m = gate_fast(x.m, rm * rm, ndt, rate_m);
+            x.m = gate_fast(x.m, rcp_near(em * em), ndt, rate_m);
             x.h = gate_to(x.h, h_inf, decay(ndt, rate_h));
             x.j = gate_to(x.j, h_inf, decay(ndt, rate_j));
             ina = P.v[gna] * x.m * x.m * x.m * x.h * x.j * (u - Ena);
@@ -485,14 +493,16 @@ struct ModelTP06 {
         const T ipk = P.v[gpk] * ux * rcp(c1 + FW_EX(u - (T)25.0, -1 / 5.98));
         const T ibna = P.v[gbna] * (u - Ena);
         const T ibca = P.v[gbca] * (u - Eca);
-        // calc_irel: kCaSR = kn / ks
+        // calc_irel: kCaSR = kr = kn / ks, kn = maxsr ks - (maxsr - minsr) casr^2 as a
+        // sum without a difference
         const T cs2 = casr * casr;
         const T ks = cs2 + P.v[d_ec2];
-        const T kn = P.v[maxsr] * ks - P.v[d_dsr] * cs2;
-        const T drr = P.v[k4] * (c1 - x.rr) - P.v[k2_] * kn * rcp(ks) * cass * x.rr;
+        const T kn = P.v[minsr] * cs2 + P.v[d_mec];
+        const T kr = div_near(kn, ks);
+        const T drr = P.v[k4] * (c1 - x.rr) - P.v[k2_] * kr * cass * x.rr;
         x.rr += dt * drr;
-        const T kc = P.v[k1_] * ks * cass * cass;
-        x.oo = div_near(kc * x.rr, P.v[k3] * kn + kc);
+        const T kc = P.v[k1_] * cass * cass;
+        x.oo = div_near(kc * x.rr, P.v[k3] * kr + kc);
         const T irel = P.v[Vrel] * x.oo * (casr - cass);
         const T ileak = P.v[Vleak] * (casr - cai);
         const T cai2 = cai * cai;
@@ -504,7 +514,12 @@ struct ModelTP06 {
         const T dCaSS = dt * (irel * P.v[d_vsrss] - ixfer * P.v[d_vcss] -
                               ical * P.v[d_ssf]);
         const T dNai = -(ina + ibna + (T)3 * (inak + inaca)) * P.v[d_naf];
-        const T dKi = -(ik1 + ito + ikr + iks - (T)2 * inak + ipk) * P.v[d_naf];
+        T dKi = -(ik1 + ito + ikr + iks - (T)2 * inak + ipk);
+        // float32: the three factors one by one.  A product formed on the host
+        // is rounded once, but that rounding is an error of every increment,
+        // and adds to those of the parameters where these offset them
+        if constexpr (sizeof(T) == 4) dKi = dt * (dKi * P.v[d_icf] * P.v[CAPACITANCE]);
+        else dKi *= P.v[d_naf];
         x.casr += buffered_step(casr, P.v[Bufsr], P.v[Kbufsr], dCaSR);
         x.cass += buffered_step(cass, P.v[Bufss], P.v[Kbufss], dCaSS);
         x.nai += dNai;
