@@ -8,17 +8,20 @@
 // These forms spend few of them and leave the rest to the integer and
 // special-function units:
 //   * exp: the table-driven method of P. T. P. Tang (ACM TOMS 15, 1989) with
-//     2^(j/256): x = n ln2/256 + r, |r| < 1.4e-3 (n rounded in float32 from
-//     the high word), e^r by its series to r^4 / 24 (remainder below 4e-17),
-//     the power of two added to the exponent field: 8 float64 instructions;
+//     2^(j/256): x = n ln2/256 + r (n rounded in float32 from the high
+//     word, so |r| < 1.5e-3 for |x| < 60, < 2.1e-3 up to 700), e^r by its
+//     series to r^4 / 24 (remainder below 7e-17, 3.5e-16), the power of two
+//     added to the exponent field: 8 float64 instructions;
 //   * log: P. T. P. Tang (ACM TOMS 16, 1990) with 128 intervals: x = 2^e m,
 //     r = c_j m - 1, |r| < 4.0e-3, log1p by its series to r^6 / 6: 10;
 //   * reciprocal: rcp.approx.ftz.f64 (PTX: relative error at most 2^-20) and
 //     one step of third order, y (1 + e + e^2), e = 1 - d y: 3;
 //   * reciprocal square root: rsqrt.approx.ftz.f64 and the third-order step
 //     y (1 + e / 2 + 3 e^2 / 8), e = 1 - d y^2: 5.
-// Errors against 64-bit references: exp and the reciprocals within 1.5 ulp,
-// log within 1.5 ulp of max(1, |log x|).  Arguments are those of the models'
+// Errors against extended precision: exp within 1.5 ulp for |x| < 60 and 2.5
+// up to 700 (half an ulp each for the table and the last sum, the rest the
+// series' remainder), the reciprocals within 1.5 ulp, log within 1.5 ulp of
+// max(1, |log x|).  Arguments are those of the models'
 // in-range updates: finite, exponents of at most a few hundred, positive
 // normal numbers under log, 1 / x and 1 / sqrt(x) (log hands anything else
 // to CUDA's).

@@ -274,3 +274,17 @@ def test_float32_update_no_less_exact(lib, oracle, model, name):
         new, old = off[0][k], off[1][k]
         for f in (lambda d: np.sqrt(np.mean(d * d)), lambda d: np.quantile(d, 0.99)):
             assert f(new) <= 1.5 * f(old) + 2.0 ** -24, (k, f(new), f(old))
+
+
+@pytest.mark.skipif(np.finfo(np.longdouble).nmant < 62,
+                    reason="needs a long double wider than double")
+@pytest.mark.parametrize("span,bound", [(1.0, 1.5), (60.0, 1.5), (600.0, 2.5), (699.0, 2.5)])
+def test_float64_exponential_ulps(lib, span, bound):
+    """Units in the last place of the result: half each for the table and the
+    last sum, the series' remainder r^5 / 120 at the largest r of the range."""
+    gen = np.random.default_rng(3)
+    x = gen.uniform(-span, span, 1000000)
+    want = np.exp(x.astype(np.longdouble))
+    ulp = np.spacing(want.astype(np.float64)).astype(np.longdouble)
+    err = np.abs(_eval(lib, 0, x).astype(np.longdouble) - want) / ulp
+    assert float(err.max()) < bound
