@@ -971,15 +971,16 @@ __global__ void __launch_bounds__(kTmaNT, 1) k_batch_all(const __grid_constant__
     }
 #undef FW_BATCH_GROUP
     // the last CTA to finish zeroes the counters and fills the next
-    // launch's events (no CTA reads a description any more)
-    unsigned *done = reinterpret_cast<unsigned *>(smem);   // the stages are free
+    // launch's events (no CTA reads a description any more).  The answer goes
+    // round in the barrier, not through the stages: where a wait gave up, a
+    // copy into them may still be under way
     __syncthreads();
+    bool last = false;
     if (threadIdx.x == 0) {
         __threadfence();
-        *done = atomicAdd(&k.scratch[1], 1u);
+        last = atomicAdd(&k.scratch[1], 1u) == gridDim.x - 1;
     }
-    __syncthreads();
-    if (*done != gridDim.x - 1) return;
+    if (!__syncthreads_or(last)) return;
     if (threadIdx.x < kGroups) atomicExch(&k.scratch[2 + 2 * threadIdx.x], 0u);
     if (threadIdx.x == 0) atomicExch(&k.scratch[1], 0u);
     if (k.next_ks)
