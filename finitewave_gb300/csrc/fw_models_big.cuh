@@ -904,21 +904,21 @@ struct ModelCRN {
             // differs by 1e-3 there
             return update_ref<T>(u, un, x, P, dt);
         } else {
-            if (fabs(u) < P.v[d_lim]) return update_in_range<T>(u, un, x, P, dt);
-            return update_any<T>(u, un, x, P, dt);
+            if (fabs(u) < P.v[d_lim]) return update_in_range(u, un, x, P, dt);
+            return update_any(u, un, x, P, dt);
         }
     }
 
     // As ModelTP06::update_in_range (float64 only): one quotient per rate.
     // 192 x 190 nodes: 65 against 180 us a step.
-    template <class T>
-    __device__ static __forceinline__ T update_in_range(T u, T un, St<T> &x,
-                                                        const Params<T, NP + ND> &P,
-                                                        T dt)
+    __device__ static __forceinline__ double
+    update_in_range(double u, double un, St<double> &x,
+                    const Params<double, NP + ND> &P, double dt)
     {
         using namespace dm;
+        using T = double;
         const T c1 = (T)1;
-        const T ndt = sizeof(T) == 8 ? -dt : -dt * (T)kLog2e;
+        const T ndt = -dt;
         const T cai = (T)x.cai, nai = (T)x.nai, carel = (T)x.carel;
         const T caup = (T)x.caup, ki = (T)x.ki;
         const T rnai = rcp(nai);
@@ -1071,24 +1071,24 @@ struct ModelCRN {
                           inaca + ibna + ibca);
     }
 
-    // The update in the reference's order: float32, and float64 potentials
-    // outside the range above.
+    // The update in the reference's order, for potentials outside the range
+    // above.
     // (Copies go into the call, so that x and P keep to registers elsewhere.)
-    template <class T>
-    __device__ static __forceinline__ T update_any(T u, T un, St<T> &x,
-                                                   const Params<T, NP + ND> &P, T dt)
+    __device__ static __forceinline__ double update_any(double u, double un, St<double> &x,
+                                                        const Params<double, NP + ND> &P,
+                                                        double dt)
     {
-        St<T> y = x;
-        Params<T, NP + ND> Q = P;
-        un = update_call<T>(u, un, y, Q, dt);
+        St<double> y = x;
+        Params<double, NP + ND> Q = P;
+        un = update_call(u, un, y, Q, dt);
         x = y;
         return un;
     }
-    template <class T>
-    __device__ static __noinline__ T update_call(T u, T un, St<T> &x,
-                                                 const Params<T, NP + ND> &P, T dt)
+    __device__ static __noinline__ double update_call(double u, double un, St<double> &x,
+                                                      const Params<double, NP + ND> &P,
+                                                      double dt)
     {
-        return update_ref<T>(u, un, x, P, dt);
+        return update_ref<double>(u, un, x, P, dt);
     }
     template <class T>
     __device__ static __forceinline__ T update_ref(T u, T un, St<T> &x,
@@ -1379,8 +1379,8 @@ struct ModelLR91 {
             // differs by 1e-3 there
             return update_ref<T>(u, un, x, P, dt);
         } else {
-            if (in_range(u, u - P.v[d_ek1])) return update_in_range<T>(u, un, x, P, dt);
-            return update_any<T>(u, un, x, P, dt);
+            if (in_range(u, u - P.v[d_ek1])) return update_in_range(u, un, x, P, dt);
+            return update_any(u, un, x, P, dt);
         }
     }
     __device__ static __forceinline__ bool in_range(double u, double x)
@@ -1391,12 +1391,12 @@ struct ModelLR91 {
     // As ModelTP06::update_in_range; var + dt (inf - var) / tau with
     // tau = 1 / (a + b), inf = a / (a + b) is var + dt (a (1 - var) - b var).
     // 192 x 190 nodes: 33 against 75 us a step (float64 only).
-    template <class T>
-    __device__ static __forceinline__ T update_in_range(T u, T un, St<T> &x,
-                                                        const Params<T, NP + ND> &P,
-                                                        T dt)
+    __device__ static __forceinline__ double
+    update_in_range(double u, double un, St<double> &x,
+                    const Params<double, NP + ND> &P, double dt)
     {
         using namespace dm;
+        using T = double;
         const T c1 = (T)1;
         auto gate = [dt](T v, T a, T b) { return v + dt * (a * ((T)1 - v) - b * v); };
         // calc_ina
@@ -1469,24 +1469,24 @@ struct ModelLR91 {
         return un - dt * (ina + isi + (ik1 + ikp + ib) + ik);
     }
 
-    // The update in the reference's order: float32, and float64 potentials
-    // outside the range above.
+    // The update in the reference's order, for potentials outside the range
+    // above.
     // (Copies go into the call, so that x and P keep to registers elsewhere.)
-    template <class T>
-    __device__ static __forceinline__ T update_any(T u, T un, St<T> &x,
-                                                   const Params<T, NP + ND> &P, T dt)
+    __device__ static __forceinline__ double update_any(double u, double un, St<double> &x,
+                                                        const Params<double, NP + ND> &P,
+                                                        double dt)
     {
-        St<T> y = x;
-        Params<T, NP + ND> Q = P;
-        un = update_call<T>(u, un, y, Q, dt);
+        St<double> y = x;
+        Params<double, NP + ND> Q = P;
+        un = update_call(u, un, y, Q, dt);
         x = y;
         return un;
     }
-    template <class T>
-    __device__ static __noinline__ T update_call(T u, T un, St<T> &x,
-                                                 const Params<T, NP + ND> &P, T dt)
+    __device__ static __noinline__ double update_call(double u, double un, St<double> &x,
+                                                      const Params<double, NP + ND> &P,
+                                                      double dt)
     {
-        return update_ref<T>(u, un, x, P, dt);
+        return update_ref<double>(u, un, x, P, dt);
     }
     template <class T>
     __device__ static __forceinline__ T update_ref(T u, T un, St<T> &x,
