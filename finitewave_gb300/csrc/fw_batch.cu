@@ -930,11 +930,12 @@ __global__ void __launch_bounds__(kTmaNT, 1)
 // group, a small batch's time was the six kernels' start-up (each about 6 us
 // before its first tile) and their launches one behind the other; one
 // kernel holds six copies of the tile loop at 128 registers, of which the
-// Fenton-Karma ones spill a few (5 % slower a tile), hence the other form
-// for large batches.  One launch of four steps, measured (CUDA events):
-//   tiles        121   1016   1963   3436   28677
-//   per group   39.2   88.9  137.0  192.8   975.8 us
-//   one kernel  21.2   54.6   91.3  171.6  1035.0 us
+// Fenton-Karma ones spill a few (3 % slower in large batches), hence the
+// other form for these.  One launch of four steps, measured (CUDA events,
+// square tissues of all six groups):
+//   tiles        105    859   1753   3397   7209  10970  14411  27435  37278
+//   per group   31.1   80.5  122.6  155.0  241.8  346.4  435.5  777.4 1034.7 us
+//   one kernel  15.8   33.9   68.0  118.9  224.2  346.4  435.5  796.4 1070.9 us
 struct BatchK {
     BTissueT *tissues;
     const BTileT *tiles;
@@ -1076,7 +1077,9 @@ inline int batch_tma_attr(bool pair, cudaStream_t stream)
     return FW_OK;
 }
 
-// Tiles per CTA from which a batch runs one kernel per group.
+// Tiles per CTA from which a batch runs one kernel per group: the two forms
+// are level at 72 and 95 tiles a CTA (table at BatchK), the one kernel 7 %
+// ahead at 47 and 2.4 % behind at 180.
 constexpr int kGroupKernels = 64;
 
 static_assert(sizeof(fused::FusedK) % 16 == 0 && offsetof(BTissueT, f) % 16 == 0,
