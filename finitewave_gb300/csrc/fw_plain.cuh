@@ -265,12 +265,15 @@ constexpr int step_threads()
 // an SM 186, 110, 139, 29.0, 10.5, with 1024 131, 94, 139, 29.0, 10.5.
 constexpr int kRestThreads = 152 * 512;
 
-// CTAs of a step.  Listed steps run one node per thread; the others, bound
-// by memory, loop over the grid with the resident CTAs.
-template <class M, class T>
-constexpr int step_blocks()
+// CTAs of a step.  Listed and float64 steps run one node per thread; the
+// others loop over the grid with the resident CTAs.  Detailed float32 steps
+// without a list as well: TP06 236^3 shell (7 % myocytes) 140 us a step, 175
+// with one node per thread, Courtemanche 160^3 shell 108 against 126, TP06
+// 200 x 200 x 40 60.8 against 59.4.
+template <class T>
+constexpr int step_blocks(bool listed)
 {
-    return UseList<M, T>::value ? 1 << 26 : 152 * 8;
+    return listed || sizeof(T) == 8 ? 1 << 26 : 152 * 8;
 }
 
 template <class M, int ST, class T, bool LIST>
@@ -282,15 +285,17 @@ __global__ void __launch_bounds__(step_threads<T>(), (MinBlocks<M, T>::value))
     const int64_t n = LIST ? (int64_t)k.n_myo : k.n;
     // Steps of one call follow one another with programmatic serialisation:
     // the next one's CTAs take their places, read their parameters and wait
-    // here while this one's last CTAs run.  A listed float64 step lets them
-    // come only when a CTA is done: placed earlier, in the slots that this
-    // step's CTAs leave, they would not spread evenly over the SMs, whose
-    // float64 pipes set the time (TP06 192 x 190: 68 against 61 us a step).
-    // With and without the overlap, us a step: Courtemanche float32 511 x 387
-    // 12.8 and 14.5, Aliev-Panfilov float32 256 x 240 x 60 59.8 and 61.8 and
-    // 320 x 300 4.0 and 5.8 (ECG samples included), float64 600 x 601 with
-    // 20 % fibrosis 28.5 and 30.9.
-    constexpr bool kLate = LIST && sizeof(T) == 8;
+    // here while this one's last CTAs run.  A float64 step lets them come
+    // only when a CTA is done: placed earlier, in the slots that this step's
+    // CTAs leave, they would not spread evenly over the SMs, whose float64
+    // pipes set the time.  Us a step early and late: TP06 192 x 190 68 and 61,
+    // in grid order 100 x 100 57.8 and 33.4, Aliev-Panfilov 100 x 100 3.9 and
+    // 3.6, 130 x 140 5.9 and 3.9, 150 x 151 without a list 13.4 and 4.2,
+    // Fenton-Karma 150 x 151 without a list 35 and 11.  With and without the
+    // overlap: Courtemanche float32 511 x 387 12.8 and 14.5, Aliev-Panfilov
+    // float32 256 x 240 x 60 59.8 and 61.8 and 320 x 300 4.0 and 5.8 (ECG
+    // samples included), float64 600 x 601 with 20 % fibrosis 28.5 and 30.9.
+    constexpr bool kLate = sizeof(T) == 8;
     if constexpr (!kLate) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (k.n_up && blockIdx.x == gridDim.x - 1) {
@@ -710,10 +715,9 @@ int run_plain(const fw_step_args *a, int64_t n_begin, int64_t n_steps,
     const int threads = sizeof(T) == 4 && listed ? kListThreadsF32 : step_threads<T>();
     k.list = listed ? a->node_list : nullptr;
     k.n_myo = (int32_t)a->n_list_myo;
-    const int blocks = !listed         ? grid_for(g.n, threads, step_blocks<M, T>())
-                       : a->n_list_myo ? grid_for(a->n_list_myo, threads,
-                                                  step_blocks<M, T>())
-                                       : 0;
+    // (without a myocyte in the list, none)
+    const int64_t stepped = listed ? a->n_list_myo : g.n;
+    const int blocks = stepped ? grid_for(stepped, threads, step_blocks<T>(listed)) : 0;
     const int blocks_rest = grid_for(g.n - a->n_list_myo, threads * kRestNodes,
                                      kRestThreads / threads);
     cudaLaunchAttribute attr;
