@@ -519,9 +519,10 @@ struct ModelBO {
             const float ss = sigmoid_of(__fmul_rn(P.v[d_ks], __fsub_rn(u, P.v[u_s])));
             const float s = __fmaf_rn(bw ? P.v[d_s1] : P.v[d_s2], __fsub_rn(ss, x.s), x.s);
             x.s = s;
-            const float fi = __fmul_rn(__fmul_rn(v, __fsub_rn(u, P.v[theta_v])),
+            // (the gate first: below theta_v the product is 0 however far u is)
+            const float fi = __fmul_rn(__fmul_rn(bv ? 0.f : v, __fsub_rn(u, P.v[theta_v])),
                                        __fsub_rn(P.v[u_u], u));
-            const float r = __fmul_rn(bv ? 0.f : P.v[d_fi], fi);
+            const float r = __fmul_rn(P.v[d_fi], fi);
             const float so = sigmoid_of(__fmul_rn(P.v[d_kso], __fsub_rn(u, P.v[u_so])));
             const float out = bw ? __fmul_rn(__fsub_rn(u, P.v[u_o]),
                                              bo ? P.v[d_o1] : P.v[d_o2])

@@ -151,3 +151,19 @@ def test_fused_update(lib, index, model):
         assert np.abs(g - w).max() < 14 * 2.0 ** -24 * max(1.7, float(np.abs(w).max()))
         # the two forms differ by no more than the quotients' roundings do
         assert np.sqrt(np.mean((g - w) ** 2)) <= 1.01 * np.sqrt(np.mean((q - w) ** 2)) + 2.0 ** -40
+
+
+@pytest.mark.parametrize("model", ["BuenoOrovio2D", "MitchellSchaeffer2D", "FentonKarma2D",
+                                   "Barkley2D"])
+def test_float32_step_far_out(model):
+    """Potentials of a simulation that blows up: finite where every term of
+    the float64 step's fits float32, with its value."""
+    import finitewave_gb300 as fg
+    u = -np.logspace(1, 12 if model in ("MitchellSchaeffer2D", "Barkley2D") else 36, 200)
+    u = u.astype(np.float32).astype(np.float64)
+    m = getattr(fg, model)()
+    state = [np.full(u.size, 0.5) for _ in m._state_names]
+    got, want = _step(fg, model, "float32", u, state), _step(fg, model, "float64", u, state)
+    for g, w in zip(got, want):
+        assert np.isfinite(g).all()
+        assert np.all(np.abs(g - w) <= 1e-4 * np.maximum(1.0, np.abs(w)))
