@@ -92,7 +92,9 @@ __device__ __forceinline__ float buffered_step(float c0, float B, float K,
     return 2.f * q * dm::rcp(p + sqrtf(fmaxf(p * p + 4.f * q, 0.f)));
 }
 // float64: the root's own form (sqrt(b^2 + 4 c) - b) / 2 would cancel four
-// digits of the subspace calcium; sqrt as x / sqrt(x).
+// digits of the subspace calcium; sqrt as x / sqrt(x).  With p < 0 -- a
+// concentration below -K, or one that more than doubles in the step -- the
+// root's other form is the one without cancellation.
 __device__ __forceinline__ double buffered_step(double c0, double B, double K,
                                                 double d)
 {
@@ -100,6 +102,8 @@ __device__ __forceinline__ double buffered_step(double c0, double B, double K,
     const double p = kc + B * K * dm::rcp(kc) - d;
     const double q = kc * d;
     const double s = p * p + 4.0 * q;
+    if (__double2hiint(p) < 0 || __double2hiint(s) <= 0x00100000)
+        return 0.5 * (sqrt(s) - p);
     return 2.0 * q * dm::rcp(p + s * dm::rsq(s));
 }
 

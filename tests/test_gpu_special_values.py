@@ -157,3 +157,26 @@ def test_step_of_zero(fg, model, prec):
             # one rounding where a new value is formed as inf - (inf - x)
             eps = 2.0 ** -50 if prec == "float64" else 2.0 ** -21
             assert np.all(np.abs(got[k] - state[k]) <= eps * np.maximum(1, np.abs(state[k]))), k
+
+
+@pytest.mark.parametrize("prec", ["float64"])
+def test_calcium_far_out(fg, oracle, prec):
+    """TP06's calcium spaces from concentrations below minus their buffers'
+    constants (a simulation that blows up) and from empty ones: the root that
+    the reference-order quadratic takes."""
+    n = 400
+    gen = np.random.default_rng(2)
+    state = _state(fg, "TP062D", n)
+    state["cass"] = np.concatenate([-np.logspace(-5, 0, n // 2), np.logspace(-9, 0, n // 2)])
+    state["casr"] = np.concatenate([gen.uniform(-3, -0.01, n // 2), gen.uniform(0.01, 8, n // 2)])
+    state["rr"], state["oo"] = np.zeros(n), np.zeros(n)
+    u = np.linspace(-90, 40, n)
+    got = _node_update(fg, "TP062D", prec, u, state)
+    want = _oracle_update(oracle, "tp06", u, state)
+    for k in want:
+        w, g = want[k], got[k]
+        assert np.array_equal(np.isfinite(g), np.isfinite(w)), k
+        # the reference's own root cancels up to eight digits of a calcium
+        # of 1e-9 against its buffer of 0.4
+        fine = np.isfinite(w)
+        assert np.all(np.abs(g - w)[fine] <= 1e-9 * np.maximum(1.0, np.abs(w[fine]))), k
