@@ -520,7 +520,8 @@ struct ModelBO {
             const float s = __fmaf_rn(bw ? P.v[d_s1] : P.v[d_s2], __fsub_rn(ss, x.s), x.s);
             x.s = s;
             // (the gate first: below theta_v the product is 0 however far u is)
-            const float fi = __fmul_rn(__fmul_rn(bv ? 0.f : v, __fsub_rn(u, P.v[theta_v])),
+            const float vg = __fmul_rn(v, bv ? 0.f : 1.f);
+            const float fi = __fmul_rn(__fmul_rn(vg, __fsub_rn(u, P.v[theta_v])),
                                        __fsub_rn(P.v[u_u], u));
             const float r = __fmul_rn(P.v[d_fi], fi);
             const float so = sigmoid_of(__fmul_rn(P.v[d_kso], __fsub_rn(u, P.v[u_so])));

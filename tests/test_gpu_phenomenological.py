@@ -167,3 +167,21 @@ def test_float32_step_far_out(model):
     for g, w in zip(got, want):
         assert np.isfinite(g).all()
         assert np.all(np.abs(g - w) <= 1e-4 * np.maximum(1.0, np.abs(w)))
+
+
+@pytest.mark.parametrize("model", MODELS)
+def test_float32_step_state_not_finite(model):
+    """A state variable that is NaN or infinite makes the same variables not
+    finite as in float64."""
+    import finitewave_gb300 as fg
+    m = getattr(fg, model)()
+    values = [np.nan, np.inf, -np.inf]
+    for u0 in (0.001, 0.05, 0.2, 0.9):
+        n = len(m._state_names) * 3
+        state = [np.full(n, 0.5) for _ in m._state_names]
+        for i in range(len(state)):
+            state[i][3 * i:3 * i + 3] = values
+        u = np.full(n, np.float32(u0), dtype=np.float64)
+        for g, w in zip(_step(fg, model, "float32", u, state),
+                        _step(fg, model, "float64", u, state)):
+            assert np.array_equal(np.isfinite(g), np.isfinite(w))
