@@ -223,6 +223,21 @@ __device__ __forceinline__ double ex(double x)
     return ex_scaled(x, 1.0, (float)(256 * kLog2e));
 }
 
+// Whether all are finite; whether all are positive, normal and finite.  On
+// the bits, beside the float64 pipe.
+template <class... A>
+__device__ __forceinline__ bool all_finite(A... a)
+{
+    int m = 0;
+    ((m = max(m, __double2hiint(a) & 0x7fffffff)), ...);
+    return m < 0x7ff00000;
+}
+template <class... A>
+__device__ __forceinline__ bool all_normal(A... a)
+{
+    return (((unsigned)(__double2hiint(a) - 0x00100000) < 0x7fe00000u) && ...);
+}
+
 // x limited to [-690, 690], on the bits; a NaN (quiet, as arithmetic makes
 // them: its high word is above infinity's) stays one
 __device__ __forceinline__ double limited(double x)

@@ -310,8 +310,10 @@ struct ModelTP06 {
         const T Ek = P.v[RTONF] * dm::lg(dm::quotient(P.v[ko], (T)x.Ki));
         // the range in which no exponential or product of them below leaves
         // T's (the squares (u + 25)^2 / 170 and the like set |u| < 300, which
-        // is d_lim for parameters as they come)
-        if (in_range(u, u - Ek, P.v[d_lim])) return update_in_range<T>(u, un, x, P, dt, Ek);
+        // is d_lim for parameters as they come), and states with which no
+        // infinity meets a 0 in a product that a quotient would not have
+        if (in_range(u, u - Ek, P.v[d_lim]) && regular(x))
+            return update_in_range<T>(u, un, x, P, dt, Ek);
         return update_any<T>(u, un, x, P, dt);
     }
     __device__ static __forceinline__ bool in_range(double u, double x, double lim)
@@ -322,6 +324,16 @@ struct ModelTP06 {
     {
         return fabsf(u) < fminf(lim, 130.f) && x > -100.f && x < 1000.f;
     }
+    __device__ static __forceinline__ bool regular(const St<double> &x)
+    {
+        return dm::all_normal((double)x.cai, (double)x.nai, (double)x.Ki) &&
+               dm::all_finite((double)x.casr, (double)x.cass, x.m, x.h, x.j, x.xr1, x.xr2,
+                              x.xs, x.r, x.s, x.d, x.f, x.f2, x.fcass, x.rr, x.oo);
+    }
+    // (float32: an infinite calcium, whose currents make the potential
+    // infinite or NaN in this step in any form, is not looked for: 1 % of a
+    // step)
+    __device__ static __forceinline__ bool regular(const St<float> &) { return true; }
 
     // The update with few divisions and exponentials, in either precision:
     // every rate is written as one quotient -- 1 / (1 + e^-y) as e^y / (1 + e^y),
@@ -908,9 +920,17 @@ struct ModelCRN {
             // differs by 1e-3 there
             return update_ref<T>(u, un, x, P, dt);
         } else {
-            if (fabs(u) < P.v[d_lim]) return update_in_range(u, un, x, P, dt);
+            if (fabs(u) < P.v[d_lim] && regular(x)) return update_in_range(u, un, x, P, dt);
             return update_any(u, un, x, P, dt);
         }
+    }
+
+    __device__ static __forceinline__ bool regular(const St<double> &x)
+    {
+        return dm::all_normal((double)x.nai, (double)x.ki, (double)x.cai) &&
+               dm::all_finite((double)x.caup, (double)x.carel, x.m, x.h, x.j, x.d, x.f,
+                              x.oa, x.oi, x.ua, x.ui, x.xr, x.xs, x.fca, x.irel, x.vrel,
+                              x.urel, x.wrel);
     }
 
     // As ModelTP06::update_in_range (float64 only): one quotient per rate.

@@ -180,3 +180,25 @@ def test_calcium_far_out(fg, oracle, prec):
         # of 1e-9 against its buffer of 0.4
         fine = np.isfinite(w)
         assert np.all(np.abs(g - w)[fine] <= 1e-9 * np.maximum(1.0, np.abs(w[fine]))), k
+
+
+@pytest.mark.parametrize("model,name", [
+    ("TP062D", "tp06"), ("Courtemanche2D", "crn"), ("LuoRudy912D", "lr91")])
+def test_states_not_finite(fg, oracle, model, name):
+    """One state variable of a node infinite, NaN, 0 or negative (a simulation
+    that blows up): the others are finite where the reference-order update's
+    are."""
+    m = getattr(fg, model)()
+    values = [np.inf, -np.inf, np.nan, 0.0, -0.5]
+    names = list(m._state_names)
+    n = len(names) * len(values)
+    state = _state(fg, model, n)
+    for i, k in enumerate(names):
+        state[k][i * len(values):(i + 1) * len(values)] = values
+    u = np.full(n, -31.25)
+    got = _node_update(fg, model, "float64", u, state)
+    want = _oracle_update(oracle, name, u, state)
+    for k in want:
+        ok = np.isfinite(got[k]) | ~np.isfinite(want[k])
+        bad = [(names[i // len(values)], values[i % len(values)]) for i in np.flatnonzero(~ok)]
+        assert not bad, (k, bad)
