@@ -185,3 +185,19 @@ def test_float32_step_state_not_finite(model):
         for g, w in zip(_step(fg, model, "float32", u, state),
                         _step(fg, model, "float64", u, state)):
             assert np.array_equal(np.isfinite(g), np.isfinite(w))
+
+
+@pytest.mark.parametrize("model", MODELS)
+def test_float32_step_nan_as_float64(model):
+    """Infinite potentials and NaN, and the state after them, are NaN and
+    infinite where the float64 step's are."""
+    import finitewave_gb300 as fg
+    m = getattr(fg, model)()
+    u = np.repeat([np.nan, np.inf, -np.inf], 2)
+    state = [np.tile([0.0, 0.5], 3) for _ in m._state_names]
+    for _ in range(3):
+        got, want = _step(fg, model, "float32", u, state), _step(fg, model, "float64", u, state)
+        for g, w in zip(got, want):
+            assert np.array_equal(np.isnan(g), np.isnan(w))
+            assert np.array_equal(np.isinf(g), np.isinf(w))
+        u, state = want[0].astype(np.float64), [w.astype(np.float64) for w in want[1:]]
