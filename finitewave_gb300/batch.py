@@ -268,8 +268,8 @@ class TissueBatch:
             _ffi.call("fw_batch_run", ctypes.byref(b), scratch.data_ptr(), 0,
                       n, stream.cuda_stream)
             return
-        key = (n, b.plan, b.n_tissues, b.n_tiles, b.ksteps, b.grid,
-               scratch.data_ptr())
+        # (the plan handle whole: its groups' ends are launch arguments)
+        key = n, bytes(b), scratch.data_ptr()
         g = self._graphs.get(key)
         if g is None:
             g = torch.cuda.CUDAGraph()

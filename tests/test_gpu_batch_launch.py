@@ -66,3 +66,21 @@ def test_batch_launch_forms(fg, kernel, groups, sizes, steps):
             assert np.array_equal(getattr(m, n), getattr(r, n)), n
         a, b = (x.tracker_sequence.sequence[0] for x in (m, r))
         assert torch.equal(a._count, b._count) and torch.equal(a._activated, b._activated)
+
+
+@pytest.mark.parametrize("kernel", ["tma", "pairs"])
+def test_captured_launches_follow_the_groups(fg, kernel):
+    """Tissues exchanged for others of the same sizes: as many tissues and
+    tiles, other groups.  The captured launches of the first set are not
+    replayed for the second."""
+    batch = fg.TissueBatch(kernel=kernel)
+    for names in (["ap", "ap", "ms"], ["ap", "ms", "fk"], ["fk", "fk", "fk"]):
+        got = [_model(fg, n, True, 130, i, 21) for i, n in enumerate(names)]
+        want = [_model(fg, n, True, 130, i, 21) for i, n in enumerate(names)]
+        batch.models = got
+        batch.run()
+        for a, b in zip(got, want):
+            b.form = "fused"
+            b.run()
+            for k in ["u"] + list(a._state_names):
+                assert torch.equal(a._dev[k], b._dev[k]), (names, k)
