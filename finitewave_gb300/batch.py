@@ -310,6 +310,9 @@ class TissueBatch:
         active = [i for i in range(len(ms)) if remaining[i] > 0]
         stream = torch.cuda.current_stream(dev).cuda_stream
         tma = self.kernel in ("tma", "pairs")
+        # the copies of models that left the batch go first
+        ids = {id(m) for m in ms}
+        self._mirrors = {k: v for k, v in self._mirrors.items() if k in ids}
         mirrors = [self._mirror(m) for m in ms] if tma else None
         if tma:
             _copy_rows([c for m, mir in zip(ms, mirrors) for c in mir.copies_in(m)],

@@ -84,3 +84,20 @@ def test_captured_launches_follow_the_groups(fg, kernel):
             b.run()
             for k in ["u"] + list(a._state_names):
                 assert torch.equal(a._dev[k], b._dev[k]), (names, k)
+
+
+def test_copies_of_models_that_left(fg):
+    """A batch whose models are exchanged holds the copies of the present ones
+    only."""
+    import gc
+    batch = fg.TissueBatch(graphs=False)
+    held = []
+    for seed in range(3):
+        m = _model(fg, "ap", True, 500, seed, 3)
+        batch.models = [m]
+        batch.run()
+        del m
+        batch.models = []
+        gc.collect()
+        held.append(torch.cuda.memory_stats()["requested_bytes.all.current"])
+    assert held[2] <= held[0] and len(batch._mirrors) == 1
