@@ -340,11 +340,11 @@ struct ModelTP06 {
     // sums and products of such terms over their common denominator, rates
     // dt / tau instead of tau -- and in float64 the exponentials of one slope
     // share one evaluation (fw_math.cuh).  Against the form below (update_any,
-    // the reference's order) the same mathematics in 890
-    // instead of 2306 float64 instructions a node (192 x 190 nodes: 60 against
-    // 150 us a step, the float64 pipe 83 % busy in both) and 700 instead of
-    // 1070 float32 ones (256 x 256 x 40: 104 against 107 us, then bound by the
-    // latency of its loads).  Against 113-bit arithmetic, one step from states of
+    // the reference's order) the same mathematics in 910
+    // instead of 2306 float64 instructions a warp of nodes and step (192 x 190
+    // nodes: 61 against 150 us a step, the float64 pipe 82 % busy in both) and
+    // 850 instead of 1070 instructions in all in float32 (256 x 256 x 40: 103
+    // against 107 us, then bound by the latency of its loads).  Against 113-bit arithmetic, one step from states of
     // a tissue in activity, the rms error of every variable is at most that of
     // the reference's order (float64 m 5.25e-17 of itself against 5.46e-17,
     // oo 1.19e-16 against 1.29e-16, xs 4.7e-17 against 1.5e-16; float32 Ki
@@ -934,7 +934,7 @@ struct ModelCRN {
     }
 
     // As ModelTP06::update_in_range (float64 only): one quotient per rate.
-    // 192 x 190 nodes: 65 against 180 us a step.
+    // 192 x 190 nodes: 66 against 180 us a step.
     __device__ static __forceinline__ double
     update_in_range(double u, double un, St<double> &x,
                     const Params<double, NP + ND> &P, double dt)

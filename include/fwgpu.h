@@ -332,7 +332,9 @@ typedef struct fw_step_args {
                             in ascending order.  The steps whose cost is
                             arithmetic (float64, the detailed models) then
                             run one thread per myocyte, so no lane of a
-                            warp idles on a non-myocyte; same results       */
+                            warp idles on a non-myocyte; same results.  They
+                            do not read `myo`: a list belongs to the flags
+                            it was made from                                */
     int64_t n_list_myo;
     const float *weight_centre; /* TMA kernels, optional: the centre plane of
                             the weights, rows `pitch` apart (16-byte
@@ -365,7 +367,7 @@ FW_API int fw_version(void);
 /* sizeof of the ABI structs as compiled into the library, so a binding can
  * check its own layout: which = 0 fw_step_args, 1 fw_stim, 2 fw_at_tracker,
  * 3 fw_lat_tracker, 4 fw_probe_tracker, 5 fw_window, 6 fw_batch,
- * 7 fw_ecg_tracker, 8 fw_tip_tracker, 9 fw_tip.  0 for unknown. */
+ * 7 fw_ecg_tracker, 8 fw_tip_tracker, 9 fw_tip, 10 fw_rows.  0 for unknown. */
 FW_API size_t fw_struct_size(int32_t which);
 
 /* Number of kernels this library has launched in the process so far
