@@ -340,9 +340,9 @@ struct ModelTP06 {
     // sums and products of such terms over their common denominator, rates
     // dt / tau instead of tau -- and in float64 the exponentials of one slope
     // share one evaluation (fw_math.cuh).  Against the form below (update_any,
-    // the reference's order) the same mathematics in 910
+    // the reference's order) the same mathematics in 918
     // instead of 2306 float64 instructions a warp of nodes and step (192 x 190
-    // nodes: 61 against 150 us a step, the float64 pipe 82 % busy in both) and
+    // nodes: 61 against 150 us a step, the float64 pipe 81 and 83 % busy) and
     // 850 instead of 1070 instructions in all in float32 (256 x 256 x 40: 103
     // against 107 us, then bound by the latency of its loads).  Against 113-bit arithmetic, one step from states of
     // a tissue in activity, the rms error of every variable is at most that of
