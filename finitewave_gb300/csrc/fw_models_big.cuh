@@ -344,12 +344,13 @@ struct ModelTP06 {
     // instead of 2306 float64 instructions a warp of nodes and step (192 x 190
     // nodes: 61 against 150 us a step, the float64 pipe 81 and 83 % busy) and
     // 850 instead of 1070 instructions in all in float32 (256 x 256 x 40: 103
-    // against 107 us, then bound by the latency of its loads).  Against 113-bit arithmetic, one step from states of
-    // a tissue in activity, the rms error of every variable is at most that of
-    // the reference's order (float64 m 5.25e-17 of itself against 5.46e-17,
-    // oo 1.19e-16 against 1.29e-16, xs 4.7e-17 against 1.5e-16; float32 Ki
-    // 9.71e-15 against 9.72e-15); the subspace calcium, whose quadratic loses
-    // four digits in the reference's form, is 56 times closer.
+    // against 107 us, then bound by the latency of its loads).  Against 113-bit
+    // arithmetic, one step from states of a tissue in activity, the rms error of
+    // every variable is at most that of the reference's order (float64 m
+    // 5.25e-17 of itself against 5.46e-17, oo 1.19e-16 against 1.29e-16, xs
+    // 4.7e-17 against 1.5e-16; float32 Ki 9.71e-15 against 9.72e-15); the
+    // subspace calcium, whose quadratic loses four digits in the reference's
+    // form, is 56 times closer.
     template <class T>
     __device__ static __forceinline__ T update_in_range(T u, T un, St<T> &x,
                                                         const Params<T, NP + ND> &P,
@@ -509,8 +510,8 @@ struct ModelTP06 {
         const T ipk = P.v[gpk] * ux * rcp(c1 + FW_EX(u - (T)25.0, -1 / 5.98));
         const T ibna = P.v[gbna] * (u - Ena);
         const T ibca = P.v[gbca] * (u - Eca);
-        // calc_irel: kCaSR = kr = kn / ks, kn = maxsr ks - (maxsr - minsr) casr^2 as a
-        // sum without a difference
+        // calc_irel: kCaSR = kr = kn / ks, kn = maxsr ks - (maxsr - minsr) casr^2
+        // as a sum
         const T cs2 = casr * casr;
         const T ks = cs2 + P.v[d_ec2];
         const T kn = P.v[minsr] * cs2 + P.v[d_mec];
