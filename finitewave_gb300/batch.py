@@ -77,8 +77,8 @@ class _Mirror:
             versions = m.weights._version, m._myo_d._version
             if versions == self.versions:
                 return
-        ni, nj = m._shape()
-        stream = torch.cuda.current_stream(m._device()).cuda_stream
+        ni, nj = self.u[0].shape[0], self.nj
+        stream = torch.cuda.current_stream(self.myo.device).cuda_stream
         _ffi.call("fw_pack_rows", m.stencil.kind, m.weights.data_ptr(), ni, nj,
                   self.pitch, self.wpack.data_ptr(), self.centre.data_ptr(),
                   stream)
